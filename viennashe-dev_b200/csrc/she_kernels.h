@@ -27,6 +27,9 @@ struct SheDev {
   int64_t n_even, n_odd;
   const int32_t *even_harm, *odd_harm;
   const double *cblocks;
+  // contact k's facets to semiconductor cells, in the order its current adds them up:
+  // (ct_cell, ct_facet)[ct_ptr[k] .. ct_ptr[k + 1])
+  const int32_t *ct_ptr, *ct_cell, *ct_facet;
   // physics
   int32_t acoustic, optical, bnd_type, scaling_type;
   double rate_ac, rate_op, n_op, hbar_omega, tau;
@@ -55,7 +58,7 @@ int vk_she_normalise(const vshe::SheDev *P, int64_t n, const int64_t *rp, const 
                      const uint8_t *ins_diag, int scale, double *s_vec, double *sf, int64_t *diag_pos, int64_t *cptr,
                      int64_t *cursor, int64_t *cpos, void *tmp, size_t tmp_bytes, cudaStream_t s);
 int vk_she_finish(const vshe::SheDev *P, const vshe::FullDev *A, const double *x_red, const double *s_vec,
-                  const double *sf, int scale, double *xf, double *part, double *dens, int ncontacts, double *cur,
-                  cudaStream_t s);
+                  const double *sf, int scale, double *xf, double *part, double *dens, int ncontacts, double *contrib,
+                  double *cur, cudaStream_t s);
 int vk_she_residual_blocks(int64_t n_full);
 }

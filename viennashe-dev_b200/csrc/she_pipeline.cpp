@@ -43,7 +43,7 @@ struct SheProblem {
   void *d_tmp = nullptr; size_t tmp_bytes = 0;
   int32_t *d_err = nullptr;
   // outputs
-  double *d_xf = nullptr, *d_dens = nullptr, *d_cur = nullptr, *d_part = nullptr;
+  double *d_xf = nullptr, *d_dens = nullptr, *d_cur = nullptr, *d_contrib = nullptr, *d_part = nullptr;
   std::vector<int64_t> slab_ptr;
   std::unique_ptr<System> sys;
   std::unique_ptr<Batch> batch;
@@ -183,6 +183,29 @@ int SheProblem::create_device_pattern(Ctx &ctx) {
   UP(i32, H.even_harm); P.even_harm = i32;
   UP(i32, H.odd_harm); P.odd_harm = i32;
   UP(f64, H.cblocks); P.cblocks = f64;
+  {
+    // the facets of each contact's terminal current (terminal_current.hpp:47-105)
+    std::vector<std::vector<std::pair<int32_t, int32_t>>> of((size_t)ncontacts);
+    for (int c = 0; c < H.nc; ++c) {
+      if (H.contact[size_t(c)] < 0) continue;
+      for (int q = H.cf_ptr[size_t(c)]; q < H.cf_ptr[size_t(c) + 1]; ++q) {
+        const int f = H.cf_idx[size_t(q)], o = H.other_cell(f, c);
+        if (o >= 0 && H.is_semi(o)) of[size_t(H.contact[size_t(c)])].push_back({c, f});
+      }
+    }
+    std::vector<int32_t> ptr(1, 0), cell, facet;
+    for (const auto &list : of) {
+      for (const auto &cf : list) { cell.push_back(cf.first); facet.push_back(cf.second); }
+      ptr.push_back(int32_t(cell.size()));
+    }
+    UP(i32, ptr); P.ct_ptr = i32;
+    UP(i32, cell); P.ct_cell = i32;
+    UP(i32, facet); P.ct_facet = i32;
+    d_contrib = (double *)arena.alloc(sizeof(double) * std::max<size_t>(cell.size(), 1), e);
+    if (!d_contrib) return ctx.cuda_fail(e, "cudaMalloc she d_contrib");
+    // the lists are read by asynchronous uploads: they must outlive them
+    if ((e = cudaStreamSynchronize(ctx.stream)) != cudaSuccess) return ctx.cuda_fail(e, "upload she table");
+  }
 #undef UP
   P.n_even_nodes = int64_t(H.even_nodes.size() / 2);
   P.n_odd_nodes = int64_t(H.odd_nodes.size() / 2);
@@ -361,7 +384,7 @@ int SheProblem::assemble(Ctx &ctx, int upto) {
 
 int SheProblem::finish(Ctx &ctx) {
   FullDev A{d_frp, d_fci, d_fval, d_frhs};
-  int rc = vk_she_finish(&P, &A, sys->d_x64, d_s, d_sf, H.cfg.scale ? 1 : 0, d_xf, d_part, d_dens, ncontacts, d_cur, ctx.stream);
+  int rc = vk_she_finish(&P, &A, sys->d_x64, d_s, d_sf, H.cfg.scale ? 1 : 0, d_xf, d_part, d_dens, ncontacts, d_contrib, d_cur, ctx.stream);
   if (rc) return ctx.cuda_fail(cudaError_t(rc), "finish");
   const int nb = vk_she_residual_blocks(n_full);
   std::vector<double> part(2 * size_t(nb));
