@@ -217,8 +217,8 @@ int vshe_system_time_spmv(vshe_ctx *ctx, int64_t handle, int32_t precision, int3
  * matrix (int64 row offsets, int32 columns, FP64 values); every pointer is a caller-owned
  * DEVICE buffer (d_r of n doubles, d_norms2 of 2) on the current CUDA device.  The kernel is
  * queued on `stream` (a cudaStream_t; NULL = the default stream) and the call returns without
- * waiting.  Its scratch (one partial-sum pair per 2048 rows) is a fixed 512 KiB array in the
- * library's device image, so n is limited to 64 Mi rows (67,108,864): larger n returns
+ * waiting.  Its scratch (the blocks' partial sums) is a fixed 512 KiB array in the
+ * library's device image; n is limited to 64 Mi rows (67,108,864): larger n returns
  * VSHE_E_CAPACITY.  The first call on each device looks up that array's address and clears its
  * ticket counter, so it synchronises the device once and should come before any stream capture.  All calls share
  * the array: calls whose kernels overlap on the GPU (other streams or threads on the same
