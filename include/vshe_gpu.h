@@ -152,11 +152,13 @@ int vshe_set_spin_limit(vshe_ctx *ctx, uint64_t polls);
  * Every choice gives the same layout and results.  No reference counterpart. */
 int vshe_set_host_threads(int32_t threads);
 /* Sweep kernel of the members swept one task per CTA or cluster (VSHE_TRSV_PER_BLOCK,
- * VSHE_TRSV_PER_SYSTEM and their AUTO cases): -1 (default) times the candidates on each batch's
- * own factors before its first iteration and keeps the fastest; 0 one CTA per task with the
- * factor slices staged through shared memory by bulk copies; 2, 4 or 8 one thread-block cluster
- * of that many CTAs per task with a cluster barrier per level.  Every choice gives bitwise the same
- * results.  No reference counterpart: scheduling control of the triangular sweeps. */
+ * VSHE_TRSV_PER_SYSTEM and their AUTO cases): -1 (default) takes the kernels that keep the solved
+ * values in shared memory for whole systems and for block tasks whose rows fit it, and for the other
+ * tasks times the candidates on each batch's own factors before its first iteration and keeps the
+ * fastest; 0 one CTA per task with the factor slices staged through shared memory by bulk copies; 2, 4
+ * or 8 one thread-block cluster of that many CTAs per task with a cluster barrier per level.  Every
+ * choice gives bitwise the same results.  No reference counterpart: scheduling control of the
+ * triangular sweeps. */
 int vshe_set_task_sweep(vshe_ctx *ctx, int32_t kernel);
 int vshe_get_profile(vshe_ctx *ctx, double *ms, int64_t *counts);
 /* Autotuner record: the rows per reduction tile chosen for systems of n's size class
@@ -263,6 +265,41 @@ int vshe_layout_export(int64_t n, int64_t nnz, const int64_t *row_ptr, const int
 int vshe_layout_sweep_plan(int64_t n, int64_t nnz, const int64_t *row_ptr, const int32_t *col, const double *val,
                            const vshe_solve_opts *opts, int32_t num_sms, int64_t *counts, int32_t *tasks,
                            int64_t *chunks, int32_t *sdesc);
+
+/* The local part of the same plan: the block tasks whose solved values fit shared memory
+ * (k_trsv_local), for tests of the stage and ring bounds.
+ * - counts[0..8]: tasks, chunks, copies, bytes of chunk heads, consumer warps, ring entries, bytes of
+ *   a stage, the tasks of the plan that are neither local nor streams, 0.
+ * - tasks[8 t ..]: system, first chunk, forward chunks, chunks, forward levels, rows, ring, 0.
+ * - chunks[5 c ..]: first copy, copies, of them after the forward sweep, bytes of the former, bytes of
+ *   the latter.
+ * - copies[4 k ..]: source offset (bytes), stage offset, array (0 heads, 1 / 2 forward columns /
+ *   values, 3 input, 4 slot of every row, 5 / 6 backward columns / values, 7 forward result by slot,
+ *   8 row of every slot, 9 inverse diagonals), bytes.
+ * - heads: per chunk int32 offsets of the operands A, B, C and of the slice descriptors, barriers to
+ *   pass, 3 unused, the warps' descriptor ranges (consumers + 1), and the descriptors (int32 column
+ *   offset, value offset, operand index, width * 64 + rows, first row's number, level, 2 unused).
+ * - fmap / bmap[n]: the number of every solver row in its task's forward and backward sweep.
+ * Call once with NULL arrays for the counts.  Host only. */
+int vshe_layout_local_plan(int64_t n, int64_t nnz, const int64_t *row_ptr, const int32_t *col, const double *val,
+                           const vshe_solve_opts *opts, int32_t num_sms, int64_t *counts, int32_t *tasks, int32_t *chunks,
+                           int64_t *copies, uint8_t *heads, int32_t *fmap, int32_t *bmap);
+/* The stream of a system swept as one task (k_trsv_stream), for tests of its bounds.
+ * - counts[0..11]: 1 if the system has one, warps, ring entries, bytes of a stage, forward chunks, 1 if
+ *   forward / backward values are read after they left the ring, chunks, step descriptors, slices,
+ *   entries that read values older than the ring, shared memory in bytes.
+ * - chunks[11 c ..]: byte offsets of its step descriptors, entries and rows; their bytes; first
+ *   operand row and their count; steps; first and count of the values older than the ring.
+ * - steps[4 k ..]: stage offsets of the slice's entries, of its rows and of its first operand, entries
+ *   stored.
+ * - recs[5 r ..]: byte offsets of its entries and rows, SELL slice (negative: empty), entries stored,
+ *   1 forward.
+ * - patch[2 p ..]: entry, and the shared-memory offset of the older value it reads; olds: the
+ *   values' numbers (the chunks' counts rounded up to even); widths[2][16]: per sweep and warp.
+ * Call once with NULL arrays for the counts.  Host only. */
+int vshe_layout_stream_plan(int64_t n, int64_t nnz, const int64_t *row_ptr, const int32_t *col, const double *val,
+                            const vshe_solve_opts *opts, int64_t *counts, int64_t *chunks, int32_t *steps, int64_t *recs,
+                            int64_t *patch, int32_t *olds, uint8_t *widths);
 
 /* ---- SHE path on the device: she::assemble + she::solve (secondary boundary) ----
  * vshe_she_create runs the host setup of the (x, H) space (energies, expansion

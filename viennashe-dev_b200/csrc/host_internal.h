@@ -57,6 +57,25 @@ struct Layout {
             const vshe_solve_opts &opts, const double *values, std::string &err);
 };
 
+// Host tables of a system's stream (k_trsv_stream): chunks and their step descriptors, the slices in
+// stream order, the values older than the ring (their numbers by chunk; the entries that read them with
+// their shared-memory offset), and the sizes of the device arrays.
+struct StreamPlan {
+  bool ok = false;
+  int nwarp = 0, ring = 0, stage = 0, nfwd = 0, keep[2] = {0, 0};
+  uint8_t width[2][16] = {{0}, {0}};
+  std::vector<StreamChunk> chunks;
+  std::vector<unsigned char> heads;
+  std::vector<StreamRec> recs;
+  std::vector<int32_t> olds;
+  std::vector<int64_t> patch;  // (entry, offset) pairs
+  int64_t ent_bytes = 0, row_bytes = 0;
+};
+struct System;
+// 0 grid-wide, 1 one task for the system, 2 tasks of preconditioner blocks (plan_sweep_tasks)
+int sweep_kind(const System &S, bool mixed);
+void plan_stream(const System &S, const Layout &L, StreamPlan &P);
+
 // One resident linear system.  The caller's CSR (and rhs) stay in the caller's order; the
 // solver works in a level-sorted solver order (perm[q] = caller row of solver row q) on
 // SELL-32 copies of A and of the incomplete factors (solver_kernels.cuh).
@@ -77,6 +96,7 @@ struct System {
   std::vector<int32_t> lgrp_lev, lgrp_blk, ugrp_lev, ugrp_blk;
   std::vector<int64_t> loff_h, uoff_h;    // SELL slot offsets of the L and U slices (host copies)
   std::vector<int64_t> lrow0_h, uslot0_h; // first solver row / slot of every L / U slice (host copies)
+  std::vector<int32_t> urow_h;            // solver row of every backward slot (host copy)
   int32_t nlevL = 0, nlevU = 0;
   int64_t nslA = 0, nslL = 0, nslU = 0;     // SELL slices
   int64_t padA = 0, padL = 0, padU = 0;     // SELL slots (incl. padding)
@@ -102,6 +122,16 @@ struct System {
   void *d_lval = nullptr, *d_uval = nullptr, *d_udinv = nullptr;
   double *d_ytmp = nullptr;
   void *kv[9] = {nullptr};  // x r rh p v s t ph sh (FP64, solver order, n + kVecPad entries; entry n stays 0)
+  // the stream of a system swept as one task (d_stream == nullptr: none)
+  StreamPlan stream;
+  StreamChunk *d_stream = nullptr;
+  unsigned char *d_stream_heads = nullptr, *d_stream_ent = nullptr, *d_stream_row = nullptr;
+  StreamRec *d_stream_recs = nullptr;
+  int32_t *d_stream_olds = nullptr;
+  int64_t *d_stream_patch = nullptr;
+  double *d_yslot = nullptr;
+  int build_stream(Ctx &ctx, const Layout &Lt);
+  int fill_stream(Ctx &ctx, bool all);
   int64_t tile_rows = 0;    // rows per reduction tile (0: not chosen yet; see Batch::autotune_tiles)
 
   int create(Ctx &ctx, int64_t n, int64_t nnz, const int64_t *rp, const int32_t *ci, const double *v,
@@ -128,6 +158,14 @@ struct System {
 // Sweep plan of a batch: per member 0 (grid-wide sweep), 1 (one task for the system) or 2 (tasks of
 // preconditioner blocks); the tasks, the chunks of their levels, the chunks' slice descriptors,
 // and the level slice ranges of the cluster sweeps.
+// Local tasks of a batch (LocTask, k_trsv_local): the tables the kernel reads and its launch shape.
+struct LocalPlan {
+  std::vector<LocTask> tasks;
+  std::vector<LocChunk> chunks;
+  std::vector<LocCopy> copies;
+  std::vector<unsigned char> heads;
+  int consumers = 0, ring = 0, stage = 0;
+};
 struct SweepPlan {
   std::vector<char> on_task;
   std::vector<TaskDev> tasks;
@@ -137,6 +175,14 @@ struct SweepPlan {
   std::vector<int64_t> clv;
   int64_t tune_key_tasks = 0;
   bool has_tune_key = false;
+  // `tasks` in this order: those of k_trsv_task or k_trsv_cluster, local ones (k_trsv_local), streams
+  // (k_trsv_stream)
+  int nrest = 0, nlocal = 0;
+  LocalPlan local;
+  std::vector<char> own_kernel;  // 1: no task of this member is among the first nrest
+  // per member with local block tasks: the task numbers of its rows in the forward and of their slots
+  // in the backward sweep, by solver row
+  std::vector<std::vector<int32_t>> fmap, bmap;
 };
 void plan_sweep_tasks(const std::vector<System *> &sys, bool mixed, bool has_pc, int64_t num_sms, SweepPlan &plan);
 
@@ -159,7 +205,23 @@ struct Batch {
   bool tasks_tuned = false;
   int64_t tune_key_tasks = -1, tune_key_grid = -1;  // shape classes of the task and grid-wide sweeps
   std::vector<double> task_tune_ms;    // ms per apply: staged, clusters of 2, 4, 8
+  // tasks [0, nrest) run the kernel above; the others are local tasks (trsv_local.cu) and
+  // streams (trsv_stream.cu) unless vshe_set_task_sweep names a kernel for all
+  int nrest = 0;
+  struct LocalTables {
+    int tasks = 0, consumers = 0, ring = 0, stage = 0;
+    void *d_tasks = nullptr, *d_chunks = nullptr, *d_copies = nullptr, *d_heads = nullptr, *d_sys = nullptr;
+  } local;
+  struct StreamTables {
+    int tasks = 0, nwarp = 0, smem = 0;
+    void *d_tasks = nullptr;
+  } streams;
+  std::vector<char> own_kernel;
+  int build_local(Ctx &ctx, const SweepPlan &plan);
+  bool use_local(const Ctx &ctx) const;
+  bool local_captured = false;  // use_local when the chunk's graph was captured
   int launch_tasks(Ctx &ctx, int which);
+  int launch_task_kernel(Ctx &ctx, int count, int which);
   int autotune_tasks(Ctx &ctx);
   bool grid_group = true;
   // the BiCGStab iteration chunk (check_every iterations) captured once as a CUDA graph and

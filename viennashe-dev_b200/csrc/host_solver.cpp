@@ -989,6 +989,7 @@ void System::adopt_layout(const Layout &Lt) {
   lgrp_s0 = Lt.lgrp_s0; lgrp_lev = Lt.lgrp_lev; lgrp_blk = Lt.lgrp_blk;
   ugrp_s0 = Lt.ugrp_s0; ugrp_lev = Lt.ugrp_lev; ugrp_blk = Lt.ugrp_blk;
   loff_h = Lt.loff; uoff_h = Lt.uoff;
+  urow_h = Lt.urow;
   lrow0_h.assign(Lt.lstart.begin(), Lt.lstart.end()); uslot0_h.assign(Lt.ustart.begin(), Lt.ustart.end());
   nlevL = Lt.nlevL; nlevU = Lt.nlevU; nslA = Lt.nslA; nslL = Lt.nslL; nslU = Lt.nslU;
   padA = Lt.padA; padL = Lt.padL; padU = Lt.padU; nnzL = Lt.nnzL; nnzU = Lt.nnzU; nnzF = Lt.nnzF;
@@ -1084,8 +1085,61 @@ int System::setup_from_layout(Ctx &ctx, const Layout &Lt) {
     if ((e = cudaMemsetAsync((char *)d_udinv + tsz * size_t(n), 0, tsz * size_t(kVecPad), s)) != cudaSuccess) return ctx.cuda_fail(e, "memset");
   }
 #undef H2D
+  if (sweep_kind(*this, mixed) == 1) {
+    const int rc = build_stream(ctx, Lt);
+    if (rc) return rc;
+  }
   if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return ctx.cuda_fail(e, "upload pattern");
   return VSHE_OK;
+}
+
+int System::build_stream(Ctx &ctx, const Layout &Lt) {
+  plan_stream(*this, Lt, stream);
+  if (!stream.ok) return VSHE_OK;
+  cudaError_t e;
+  // one upload for the host tables, one buffer for what the device fills
+  std::vector<unsigned char> up;
+  auto put = [&](const void *src, size_t bytes) {
+    const size_t at = (up.size() + 255) & ~size_t(255);
+    up.resize(at + bytes);
+    if (bytes) std::memcpy(up.data() + at, src, bytes);
+    return at;
+  };
+  up.reserve(sizeof(StreamChunk) * stream.chunks.size() + stream.heads.size() + sizeof(StreamRec) * stream.recs.size() + 4 * stream.olds.size() +
+             8 * stream.patch.size() + 5 * 256);
+  const size_t chunks = put(stream.chunks.data(), sizeof(StreamChunk) * stream.chunks.size()), heads = put(stream.heads.data(), stream.heads.size()),
+               recs = put(stream.recs.data(), sizeof(StreamRec) * stream.recs.size()), olds = put(stream.olds.data(), 4 * stream.olds.size()),
+               patch = put(stream.patch.data(), 8 * stream.patch.size());
+  unsigned char *t = (unsigned char *)arena.alloc(up.size() + 256, e);
+  if (!t) return ctx.cuda_fail(e, "cudaMalloc stream tables");
+  if ((e = cudaMemcpyAsync(t, up.data(), up.size(), cudaMemcpyHostToDevice, ctx.stream)) != cudaSuccess) return ctx.cuda_fail(e, "upload stream tables");
+  const size_t row = size_t(stream.ent_bytes + 255) & ~size_t(255), ys = (row + size_t(stream.row_bytes) + 255) & ~size_t(255),
+               bytes = ys + sizeof(double) * size_t(n + kVecPad);
+  unsigned char *f = (unsigned char *)arena.alloc(bytes, e);
+  if (!f) return ctx.cuda_fail(e, "cudaMalloc stream");
+  if ((e = cudaMemsetAsync(f + ys, 0, bytes - ys, ctx.stream)) != cudaSuccess) return ctx.cuda_fail(e, "memset");
+  d_stream = (StreamChunk *)(t + chunks);
+  d_stream_heads = t + heads;
+  d_stream_recs = (StreamRec *)(t + recs);
+  d_stream_olds = (int32_t *)(t + olds);
+  d_stream_patch = (int64_t *)(t + patch);
+  d_stream_ent = f;
+  d_stream_row = f + row;
+  d_yslot = (double *)(f + ys);
+  const int rc = fill_stream(ctx, true);
+  if (rc) return rc;
+  // (the upload's source goes with this call)
+  if ((e = cudaStreamSynchronize(ctx.stream)) != cudaSuccess) return ctx.cuda_fail(e, "stream tables");
+  return VSHE_OK;
+}
+
+// all: the stream's tables (once); otherwise the factor's values (after every factorisation).
+int System::fill_stream(Ctx &ctx, bool all) {
+  std::vector<char> sd(vk_sysdev_size());
+  fill_sysdev(sd.data());
+  const int rc = vk_stream_fill(mixed ? 1 : 0, sd.data(), int(stream.recs.size()), d_stream_recs, d_dpos, stream.ring, int(stream.patch.size() / 2),
+                                d_stream_patch, all ? 1 : 0, d_stream_ent, d_stream_row, ctx.stream);
+  return rc ? ctx.cuda_fail(cudaError_t(rc), "stream fill") : VSHE_OK;
 }
 
 void System::fill_sysdev(void *out) const {
@@ -1118,6 +1172,390 @@ int Batch::sync_spin_limit(Ctx &ctx) {
   return VSHE_OK;
 }
 
+// The sweep of one member: 0 grid-wide, 1 one task, 2 tasks of blocks (the rule below plan_sweep_tasks
+// explains).
+int sweep_kind(const System &S, bool mixed) {
+  constexpr int64_t kCtaRowsPerLevel = 4096;
+  constexpr int32_t kCtaMinLevels = 32;
+  constexpr int64_t kTaskMaxRows = int64_t(1) << 18;
+  constexpr double kTaskBytesPerUs = 3.0e4, kGridBytesPerUs = 3.0e6, kGridLevelUs = 4.0;
+  if (S.opts.precond == VSHE_PRECOND_NONE) return 0;
+  const int mode = S.opts.trsv_mode;
+  int32_t nb = 0;
+  for (int32_t b : S.blk) nb = std::max(nb, b + 1);
+  std::vector<int64_t> bsz((size_t)nb, 0);
+  for (int32_t b : S.blk) bsz[size_t(b)]++;
+  const int64_t bmax = nb ? *std::max_element(bsz.begin(), bsz.end()) : 0;
+  const double apply_bytes = double(4 + (mixed ? 4 : 8)) * double(S.padL + S.padU) + 40.0 * double(S.n);
+  const bool one_sm_sooner = apply_bytes / kTaskBytesPerUs < kGridLevelUs * double(S.nlevL + S.nlevU) + apply_bytes / kGridBytesPerUs;
+  const bool per_sys = S.nlevL > kCtaMinLevels && S.n / std::max(S.nlevL, 1) < kCtaRowsPerLevel && one_sm_sooner;
+  const bool per_blk = (S.opts.precond == VSHE_PRECOND_BLOCK_ILU0 || S.opts.precond == VSHE_PRECOND_ILUT) && nb >= 2 && bmax <= kTaskMaxRows;
+  if (mode == VSHE_TRSV_PER_SYSTEM) return 1;
+  if (mode == VSHE_TRSV_PER_BLOCK) return 2;
+  if (mode == VSHE_TRSV_AUTO) return per_blk ? 2 : per_sys ? 1 : 0;
+  return 0;
+}
+
+// Bytes of a chunk head with its warp ranges and slice descriptors.
+static int64_t local_head_bytes(int consumers, int64_t ns) {
+  return ((int64_t(sizeof(LocHead)) + 4 * (consumers + 1) + 15) & ~int64_t(15)) + int64_t(sizeof(SliceLoc)) * ns;
+}
+
+// Appends the chunks of the sweep plan's task t to a local plan (LocTask in solver_kernels.cuh).
+static void add_local_task(const std::vector<System *> &sys, int vb, SweepPlan &P, size_t t, int64_t m) {
+  LocalPlan &L = P.local;
+  const ClusterTask &c = P.ctasks[t];
+  const System *S = sys[size_t(c.sys)];
+  std::vector<int32_t> &fm = P.fmap[size_t(c.sys)], &bm = P.bmap[size_t(c.sys)];
+  if (fm.empty()) { fm.assign(size_t(S->n), kLocPad); bm.assign(size_t(S->n), kLocPad); }
+  const int C = L.consumers;
+  LocTask T{c.sys, int32_t(L.chunks.size()), 0, 0, c.nlevL, std::max(c.nlevL, c.nlevL + c.nlevU - 1), int32_t(m), L.ring};
+  for (int pass = 0; pass < 2; ++pass) {
+    const bool lower = pass == 0;
+    const std::vector<int64_t> &off = lower ? S->loff_h : S->uoff_h, &rs = lower ? S->lrow0_h : S->uslot0_h;
+    const int64_t *lv = P.clv.data() + (lower ? c.offL : c.offU);
+    const int32_t nlev = lower ? c.nlevL : c.nlevU, lev0 = lower ? 0 : c.nlevL;
+    // operand bytes per row or slot: FP64 operand, int32 target, inverse diagonal (backward)
+    const int64_t row_bytes = lower ? 12 : 12 + vb;
+    // the chunk being filled: its slices with their warps, operand runs (aligned row ranges), slot runs
+    struct Item { SliceLoc d; int warp; };
+    std::vector<Item> items;
+    std::vector<std::pair<int64_t, int64_t>> runs, slots;
+    int64_t nslot = 0, nop = 0, last_end = -1, loc = 0;
+    int32_t lmax = 0;
+    auto flush = [&](bool last) {
+      if (items.empty()) return;
+      const int64_t ns = int64_t(items.size()), hb = local_head_bytes(C, ns), offcol = hb, offval = offcol + 4 * nslot, offA = offval + vb * nslot,
+                    offB = offA + 8 * nop, offC = offB + 4 * nop;
+      std::stable_sort(items.begin(), items.end(), [](const Item &x, const Item &y) { return x.warp < y.warp; });
+      const size_t h0 = L.heads.size();
+      L.heads.resize(h0 + size_t(hb), 0);
+      const LocHead H{int32_t(offA), int32_t(offB), int32_t(offC), int32_t(hb - int64_t(sizeof(SliceLoc)) * ns),
+                      last && lower ? c.nlevL : lmax, {0, 0, 0}};
+      std::memcpy(L.heads.data() + h0, &H, sizeof(H));
+      std::vector<int32_t> wptr((size_t)C + 1, 0);
+      for (const Item &it : items) wptr[size_t(it.warp) + 1]++;
+      for (int w = 0; w < C; ++w) wptr[size_t(w) + 1] += wptr[size_t(w)];
+      std::memcpy(L.heads.data() + h0 + sizeof(H), wptr.data(), 4 * wptr.size());
+      for (int64_t k = 0; k < ns; ++k) {
+        SliceLoc d = items[size_t(k)].d;
+        d.val = int32_t(offval + int64_t(d.col) * vb);
+        d.col = int32_t(offcol + int64_t(d.col) * 4);
+        std::memcpy(L.heads.data() + h0 + size_t(H.offD) + size_t(k) * sizeof(SliceLoc), &d, sizeof(d));
+      }
+      LocChunk ch{int32_t(L.copies.size()), 0, 0, 0, 0};
+      auto copy = [&](int kind, int64_t src, int64_t dst, int64_t bytes) {
+        if (bytes <= 0) return;
+        L.copies.push_back({src, int32_t(dst), int32_t(kind << 24 | int(bytes))});
+        ch.bytes += int32_t(bytes);
+      };
+      copy(kLocHead, int64_t(h0), 0, hb);
+      int64_t at = 0;
+      for (auto &r : slots) {
+        copy(lower ? kLocLCol : kLocUCol, 4 * r.first, offcol + 4 * at, 4 * (r.second - r.first));
+        copy(lower ? kLocLVal : kLocUVal, vb * r.first, offval + vb * at, vb * (r.second - r.first));
+        at += r.second - r.first;
+      }
+      at = 0;
+      for (auto &r : runs) {
+        const int64_t k = r.second - r.first;
+        if (lower) {
+          copy(kLocIn, 8 * r.first, offA + 8 * at, 8 * k);
+          copy(kLocFSlot, 4 * r.first, offB + 4 * at, 4 * k);
+        } else {
+          copy(kLocURow, 4 * r.first, offB + 4 * at, 4 * k);
+          copy(kLocUDinv, vb * r.first, offC + vb * at, vb * k);
+        }
+        at += k;
+      }
+      if (!lower) {
+        const int32_t early = ch.bytes;
+        const size_t n0 = L.copies.size();
+        at = 0;
+        for (auto &r : runs) { copy(kLocYSlot, 8 * r.first, offA + 8 * at, 8 * (r.second - r.first)); at += r.second - r.first; }
+        ch.nlate = int32_t(L.copies.size() - n0);
+        ch.late_bytes = ch.bytes - early;
+        ch.bytes = early;
+      }
+      ch.nrec = int32_t(L.copies.size()) - ch.rec0;
+      L.chunks.push_back(ch);
+      items.clear(); runs.clear(); slots.clear();
+      nslot = nop = 0;
+      last_end = -1;
+    };
+    for (int32_t k = 0; k < nlev; ++k) {
+      const int64_t a = lv[2 * k], b = lv[2 * k + 1];
+      for (int64_t j = a; j < b; ++j) {
+        const int64_t r0 = rs[size_t(j)], r1 = rs[size_t(j) + 1], w = off[size_t(j) + 1] - off[size_t(j)];
+        for (int tries = 0; tries < 2; ++tries) {
+          // operand entries this slice adds: its rows extend the last run, or start a new aligned one
+          const bool extend = last_end == r0;
+          const int64_t e1 = (r1 + 3) & ~int64_t(3), e0 = extend ? runs.back().second : (r0 & ~int64_t(3));
+          const int64_t add = std::max<int64_t>(e1 - e0, 0);
+          if (tries == 0 && local_head_bytes(C, int64_t(items.size()) + 1) + (4 + vb) * (nslot + w) + row_bytes * (nop + add) > L.stage) {
+            flush(false);
+            continue;
+          }
+          if (extend) runs.back().second = std::max(runs.back().second, e1);
+          else runs.push_back({e0, e1});
+          const int64_t op = nop + add - (runs.back().second - r0);
+          if (!slots.empty() && slots.back().second == off[size_t(j)]) slots.back().second += w;
+          else if (w > 0) slots.push_back({off[size_t(j)], off[size_t(j)] + w});
+          const SliceLoc d{int32_t(nslot), 0, int32_t(op), int32_t((w >> 5) << 6 | (r1 - r0)), int32_t(loc), lev0 + k, {0, 0}};
+          items.push_back({d, int((j - a) % C)});
+          nslot += w;
+          nop += add;
+          last_end = r1;
+          lmax = lev0 + k;
+          break;
+        }
+        for (int64_t r = r0; r < r1; ++r) {
+          if (lower) fm[size_t(r)] = int32_t(loc + r - r0);
+          else bm[size_t(S->urow_h[size_t(r)])] = int32_t(loc + r - r0);
+        }
+        loc += r1 - r0;
+      }
+    }
+    flush(true);
+    if (lower) T.nfwd = int32_t(L.chunks.size()) - T.c0;
+  }
+  T.nchunk = int32_t(L.chunks.size()) - T.c0;
+  L.tasks.push_back(T);
+}
+
+// Splits the tasks by kernel.  Whole systems with a stream take k_trsv_stream.  A block task whose
+// rows all fit the ring of shared memory is local (k_trsv_local); one stage size serves the batch:
+// 32 KB, or what its widest slice needs up to 64 KB, and the ring is the largest power of two
+// beside the stages (16384 values with 32 KB stages).  Larger blocks (energy slabs of large 2D
+// meshes) keep k_trsv_task: the colours of a block spread a row's neighbours over the whole slab.
+static void plan_local_tasks(const std::vector<System *> &sys, bool mixed, SweepPlan &P) {
+  const int vb = mixed ? 4 : 8;
+  const size_t nt = P.tasks.size();
+  P.nrest = int(nt);
+  P.nlocal = 0;
+  P.own_kernel.assign(sys.size(), 0);
+  P.fmap.assign(sys.size(), {});
+  P.bmap.assign(sys.size(), {});
+  P.local = LocalPlan{};
+  if (nt == 0) return;
+  struct Info { int64_t m = 0, stage = 0; double slices = 0, levels = 0; };
+  std::vector<Info> info(nt);
+  int64_t stage = 32768;
+  for (size_t t = 0; t < nt; ++t) {
+    const ClusterTask &c = P.ctasks[t];
+    const System *S = sys[size_t(c.sys)];
+    if (P.on_task[size_t(c.sys)] != 2) continue;
+    Info &I = info[t];
+    for (int pass = 0; pass < 2; ++pass) {
+      const bool lower = pass == 0;
+      const std::vector<int64_t> &off = lower ? S->loff_h : S->uoff_h, &rs = lower ? S->lrow0_h : S->uslot0_h;
+      const int64_t *lv = P.clv.data() + (lower ? c.offL : c.offU);
+      for (int32_t k = 0; k < (lower ? c.nlevL : c.nlevU); ++k) {
+        const int64_t a = lv[2 * k], b = lv[2 * k + 1];
+        for (int64_t j = a; j < b; ++j) {
+          const int64_t nr = rs[size_t(j) + 1] - rs[size_t(j)];
+          I.stage = std::max(I.stage, local_head_bytes(kLocWide, 1) + (4 + vb) * (off[size_t(j) + 1] - off[size_t(j)]) + (nr + 6) * (12 + vb));
+        }
+        if (lower) I.m += rs[size_t(b)] - rs[size_t(a)];
+        I.slices += double(b - a);
+        I.levels += 1;
+      }
+    }
+    if (I.stage <= kTaskStageBytes) stage = std::max(stage, (I.stage + 1023) & ~int64_t(1023));
+  }
+  int64_t ring = 1, need = 32;
+  while (local_smem_bytes(2 * ring, stage) <= kLocSmemMax) ring *= 2;
+  std::vector<char> kind(nt, 0);  // 0 neither, 1 local, 2 stream
+  double slices = 0, levels = 0;
+  for (size_t t = 0; t < nt; ++t) {
+    const Info &I = info[t];
+    const size_t k = size_t(P.ctasks[t].sys);
+    if (P.on_task[k] == 1) { kind[t] = sys[k]->stream.ok ? 2 : 0; continue; }
+    if (I.stage > stage || I.m > ring) continue;
+    kind[t] = 1;
+    while (need < I.m) need *= 2;
+    slices += I.slices;
+    levels += I.levels;
+  }
+  std::vector<TaskDev> tk;
+  std::vector<ClusterTask> ct;
+  std::vector<size_t> order;
+  for (int part = 0; part < 3; ++part)
+    for (size_t t = 0; t < nt; ++t)
+      if (kind[t] == part) { tk.push_back(P.tasks[t]); ct.push_back(P.ctasks[t]); order.push_back(t); }
+  P.nrest = int(std::count(kind.begin(), kind.end(), 0));
+  P.nlocal = int(std::count(kind.begin(), kind.end(), 1));
+  P.tasks.swap(tk);
+  P.ctasks.swap(ct);
+  std::fill(P.own_kernel.begin(), P.own_kernel.end(), 1);
+  for (int t = 0; t < P.nrest; ++t) P.own_kernel[size_t(P.ctasks[size_t(t)].sys)] = 0;
+  P.local.ring = int(need);
+  P.local.stage = int(stage);
+  // a little more warps than the slices of an average level, so that a level is one slice per warp
+  // and few warps only keep the level barrier company
+  P.local.consumers = 3;
+  while (P.local.consumers < kLocWide && double(P.local.consumers) < 1.1 * slices / std::max(levels, 1.0))
+    P.local.consumers = 2 * P.local.consumers + 1;
+  for (int t = P.nrest; t < P.nrest + P.nlocal; ++t) add_local_task(sys, vb, P, size_t(t), info[order[size_t(t)]].m);
+}
+
+// The stream of a system swept as one task: the slices of each level dealt to nwarp warps in steps, the
+// steps cut into chunks.  A warp's slices of a sweep are stored at one width, their widest's (the
+// kernel's variant for it; a level's slices come widest first, so the later warps get narrow ones);
+// beyond kStreamW a slice keeps its own.  No stream where a slice does not fit a stage or three
+// consecutive chunks or levels do not fit the ring.
+void plan_stream(const System &S, const Layout &L, StreamPlan &P) {
+  P = StreamPlan{};
+  const int eb = S.mixed ? int(sizeof(StreamEnt<float>)) : int(sizeof(StreamEnt<double>));
+  double slices = 0, levels = 0;
+  for (int pass = 0; pass < 2; ++pass) {
+    const std::vector<int64_t> &lv = pass == 0 ? S.lvsL : S.lvsU;
+    slices += double(lv.empty() ? 0 : lv.back() - lv.front());
+    levels += double(lv.empty() ? 0 : lv.size() - 1);
+  }
+  if (levels == 0 || S.n >= (int64_t(1) << 30)) return;
+  // one slice per warp on most levels: fewer warps make the barrier cheaper, more steps per level cost more
+  P.nwarp = 1;
+  while (P.nwarp < kStreamWarps && double(P.nwarp) < 0.95 * slices / levels) P.nwarp = std::min(2 * P.nwarp, kStreamWarps);
+  int64_t most = 0;  // entries of the widest slice
+  for (int pass = 0; pass < 2; ++pass) {
+    const std::vector<int64_t> &off = pass == 0 ? S.loff_h : S.uoff_h, &lv = pass == 0 ? S.lvsL : S.lvsU;
+    int64_t widest[kStreamWarps] = {0};
+    for (size_t k = 0; k + 1 < lv.size(); ++k)
+      for (int64_t j = lv[k]; j < lv[k + 1]; ++j) {
+        int64_t &w = widest[(j - lv[k]) % P.nwarp];
+        w = std::max(w, (off[size_t(j) + 1] - off[size_t(j)]) >> 5);
+      }
+    for (int w = 0; w < P.nwarp; ++w) {
+      P.width[pass][w] = uint8_t(stream_width(int(std::min<int64_t>(widest[w], 1 << 20))));
+      most = std::max(most, widest[w]);
+    }
+  }
+  // bytes of a chunk of so many steps, entries per lane, slices, older values and rows, with the padding
+  // step, the two descriptors past the end and the empty slice; lanes past a slice's last row
+  // read operands up to 31 rows further
+  auto bytes = [&](int64_t steps, int64_t entries, int64_t count, int64_t old, int64_t rows) {
+    return int64_t(sizeof(StreamStep)) * (steps + 3) * P.nwarp + 32 * eb * (entries + kStreamW) + 32 * int64_t(sizeof(StreamRow)) * (count + 1) +
+           8 * (rows + 8) + 8 * (old + 2) + 256;
+  };
+  // the stages take what a full ring leaves; wider slices (ILUT) take 64 KB and a smaller ring
+  P.ring = 32;  // (the stages behind it start on 128 bytes)
+  while (P.ring < S.n && P.ring < kStreamRing) P.ring *= 2;
+  const int64_t one = bytes(1, most, 1, 0, 32);
+  P.stage = int((kLocSmemMax - 128 - 8 * kStreamRing) / kLocStages & ~int64_t(1023));
+  if (one > P.stage) {
+    P.stage = 65536;
+    while (P.ring > 32 && local_smem_bytes(P.ring, P.stage) > kLocSmemMax) P.ring /= 2;
+  }
+  if (one > P.stage) return;
+  bool fits = true;
+  for (int pass = 0; pass < 2; ++pass) {
+    const bool lower = pass == 0;
+    const std::vector<int64_t> &off = lower ? S.loff_h : S.uoff_h, &rs = lower ? S.lrow0_h : S.uslot0_h, &lv = lower ? S.lvsL : S.lvsU;
+    const std::vector<int32_t> &col = lower ? L.lcol : L.ucol;
+    const size_t first = P.chunks.size();
+    std::vector<int64_t> start;  // number of each chunk's first row
+    auto stored = [&](int64_t j, int64_t warp) -> int64_t {
+      const int w = P.width[pass][warp];
+      return w > kStreamW ? std::max<int64_t>((off[size_t(j) + 1] - off[size_t(j)]) >> 5, kStreamW) : w;
+    };
+    struct Item { int64_t slice, step, warp; };
+    struct Old { int64_t item, entry; int32_t number; };  // entry: within its slice
+    std::vector<Item> items;  // of the chunk being filled
+    std::vector<Old> old;
+    int64_t steps = 0, ents = 0;  // its steps, and the entries per lane of its slices
+    auto flush = [&]() {
+      if (steps == 0) return;
+      StreamChunk c{};
+      c.nstep = int32_t((steps + 1) & ~int64_t(1));
+      c.op0 = int32_t(rs[size_t(items.front().slice)] & ~int64_t(3));
+      c.nop = int32_t(((rs[size_t(items.back().slice) + 1] + 3) & ~int64_t(3)) - c.op0);
+      c.head = int64_t(P.heads.size());
+      c.head_bytes = int32_t(sizeof(StreamStep)) * (c.nstep + 2) * P.nwarp;
+      c.ent = P.ent_bytes;
+      c.row = P.row_bytes;
+      c.ent_bytes = int32_t(32 * eb * (ents + kStreamW));
+      c.row_bytes = int32_t(32 * sizeof(StreamRow) * (items.size() + 1));
+      c.old0 = int32_t(P.olds.size());
+      c.nold = int32_t((old.size() + 1) & ~size_t(1));  // the operands after them start on 16 bytes
+      const int32_t at_row = c.head_bytes + c.ent_bytes, at_old = at_row + c.row_bytes, at_op = at_old + 8 * c.nold;
+      P.heads.resize(P.heads.size() + size_t(c.head_bytes));
+      StreamStep *d = (StreamStep *)(P.heads.data() + c.head);
+      std::fill(d, d + int64_t(c.nstep + 2) * P.nwarp, StreamStep{c.head_bytes, at_row, at_op, kStreamW});
+      P.recs.push_back(StreamRec{c.ent, c.row, -1, kStreamW, lower ? 1 : 0, 0});
+      int64_t e = 32 * eb * kStreamW, r = 32 * int64_t(sizeof(StreamRow));
+      std::vector<int64_t> at((size_t)items.size());
+      for (size_t i = 0; i < items.size(); ++i) {
+        const Item &it = items[i];
+        const int32_t w = int32_t(stored(it.slice, it.warp));
+        d[it.step * P.nwarp + it.warp] =
+            StreamStep{int32_t(c.head_bytes + e), int32_t(at_row + r), int32_t(at_op + 8 * (rs[size_t(it.slice)] - c.op0)), w};
+        P.recs.push_back(StreamRec{c.ent + e, c.row + r, int32_t(it.slice), w, lower ? 1 : 0, 0});
+        at[i] = (c.ent + e) / eb;
+        e += 32 * eb * w;
+        r += 32 * int64_t(sizeof(StreamRow));
+      }
+      const int64_t stage0 = 8 * int64_t(P.ring) + 128 + int64_t(P.chunks.size() % kLocStages) * P.stage;
+      for (size_t k = 0; k < old.size(); ++k) {
+        P.olds.push_back(old[k].number);
+        P.patch.push_back(at[size_t(old[k].item)] + old[k].entry);
+        P.patch.push_back(stage0 + at_old + 8 * int64_t(k));
+      }
+      if (old.size() & 1) P.olds.push_back(old.back().number);
+      if (!old.empty()) P.keep[pass] = 1;
+      if (at_op + 8 * int64_t(c.nop) + 256 > P.stage) fits = false;  // a step of one slice with too many older values
+      P.ent_bytes += c.ent_bytes;
+      P.row_bytes += c.row_bytes;
+      start.push_back(rs[size_t(items.front().slice)]);
+      P.chunks.push_back(c);
+      items.clear();
+      old.clear();
+      steps = ents = 0;
+    };
+    for (size_t k = 0; k + 1 < lv.size(); ++k) {
+      const int64_t end = rs[size_t(lv[k + 1])];
+      for (int64_t j = lv[k]; j < lv[k + 1];) {
+        // the step: up to nwarp slices that fit a stage on their own, with their older values
+        std::vector<Old> add;
+        int64_t e = j, sum = 0;
+        while (e < lv[k + 1] && e - j < P.nwarp) {
+          const size_t had = add.size();
+          if (end > P.ring)
+            for (int64_t q = off[size_t(e)]; q < off[size_t(e) + 1]; ++q) {
+              const int32_t c = col[size_t(q)];
+              if (c >= S.n) continue;
+              const int64_t number = lower ? int64_t(c) : L.dpos[size_t(c)];
+              if (number < end - P.ring) add.push_back(Old{e - j, q - off[size_t(e)], int32_t(number)});
+            }
+          const int64_t w = stored(e, (e - lv[k]) % P.nwarp);
+          if (e > j && bytes(1, sum + w, e + 1 - j, int64_t(add.size()), rs[size_t(e) + 1] - rs[size_t(j)]) > P.stage) { add.resize(had); break; }
+          sum += w;
+          ++e;
+        }
+        if (steps > 0 && bytes(steps + 1, ents + sum, int64_t(items.size()) + e - j, int64_t(old.size() + add.size()),
+                               rs[size_t(e)] - rs[size_t(items.front().slice)]) > P.stage) flush();
+        for (Old &o : add) { o.item += int64_t(items.size()); old.push_back(o); }
+        for (int64_t i = j; i < e; ++i) items.push_back(Item{i, steps, (i - lv[k]) % P.nwarp});
+        ++steps;
+        ents += sum;
+        j = e;
+      }
+    }
+    flush();
+    if (lower) P.nfwd = int(P.chunks.size());
+    // a value older than the ring lies in chunks before the two preceding its reader's
+    start.push_back(S.n);
+    for (size_t g = 0; first + g < P.chunks.size(); ++g)
+      if (P.keep[pass] && start[g + 1] - start[g < 2 ? 0 : g - 2] > P.ring) return;
+  }
+  if (!fits) return;
+  for (size_t k = 0; k + 1 < S.lvsL.size(); ++k)  // rows of a level and the ring
+    if (S.lrow0_h[size_t(S.lvsL[k + 1])] - S.lrow0_h[size_t(S.lvsL[k])] > P.ring) return;
+  for (size_t k = 0; k + 1 < S.lvsU.size(); ++k)
+    if (S.uslot0_h[size_t(S.lvsU[k + 1])] - S.uslot0_h[size_t(S.lvsU[k])] > P.ring) return;
+  P.ok = true;
+}
+
 // Sweep plan of a batch (host only): which members sweep as tasks (k_trsv_task, k_trsv_cluster)
 // and which in the grid-wide schedule, the tasks, the chunks of their levels with the chunks'
 // slice descriptors, and the level slice ranges of the cluster sweeps.
@@ -1135,30 +1573,12 @@ int Batch::sync_spin_limit(Ctx &ctx) {
 // grid-wide sweep costs about kGridLevelUs (its grid barrier and the latency of the level's
 // rows) on top of the apply's bytes at kGridBytesPerUs.
 void plan_sweep_tasks(const std::vector<System *> &sys, bool mixed, bool has_pc, int64_t num_sms_hint, SweepPlan &P) {
-  constexpr int64_t kCtaRowsPerLevel = 4096;
-  constexpr int32_t kCtaMinLevels = 32;
-  constexpr int64_t kTaskMaxRows = int64_t(1) << 18;
-  constexpr double kTaskBytesPerUs = 3.0e4, kGridBytesPerUs = 3.0e6, kGridLevelUs = 4.0;
   const int nsys = int(sys.size());
   std::vector<char> &on_task = P.on_task;  // 0 grid, 1 whole system, 2 per block
   on_task.assign((size_t)nsys, 0);
   if (has_pc) {
     for (int k = 0; k < nsys; ++k) {
-      const System *S = sys[size_t(k)];
-      const int mode = S->opts.trsv_mode;
-      int32_t nb = 0;
-      for (int32_t b : S->blk) nb = std::max(nb, b + 1);
-      std::vector<int64_t> bsz((size_t)nb, 0);
-      for (int32_t b : S->blk) bsz[size_t(b)]++;
-      const int64_t bmax = nb ? *std::max_element(bsz.begin(), bsz.end()) : 0;
-      const double apply_bytes = double(4 + (mixed ? 4 : 8)) * double(S->padL + S->padU) + 40.0 * double(S->n);
-      const bool one_sm_sooner = apply_bytes / kTaskBytesPerUs < kGridLevelUs * double(S->nlevL + S->nlevU) + apply_bytes / kGridBytesPerUs;
-      const bool per_sys = S->nlevL > kCtaMinLevels && S->n / std::max(S->nlevL, 1) < kCtaRowsPerLevel && one_sm_sooner;
-      const bool per_blk = (S->opts.precond == VSHE_PRECOND_BLOCK_ILU0 || S->opts.precond == VSHE_PRECOND_ILUT) && nb >= 2 &&
-                           bmax <= kTaskMaxRows;
-      if (mode == VSHE_TRSV_PER_SYSTEM) on_task[size_t(k)] = 1;
-      else if (mode == VSHE_TRSV_PER_BLOCK) on_task[size_t(k)] = 2;
-      else if (mode == VSHE_TRSV_AUTO) on_task[size_t(k)] = per_blk ? 2 : per_sys ? 1 : 0;
+      on_task[size_t(k)] = char(sweep_kind(*sys[size_t(k)], mixed));
     }
   }
   std::vector<TaskDev> &tasks = P.tasks;
@@ -1309,6 +1729,7 @@ void plan_sweep_tasks(const std::vector<System *> &sys, bool mixed, bool has_pc,
       P.has_tune_key = true;
     }
   }
+  plan_local_tasks(sys, mixed, P);
 }
 
 int Batch::build(Ctx &ctx, const std::vector<System *> &members) {
@@ -1505,7 +1926,79 @@ int Batch::build(Ctx &ctx, const std::vector<System *> &members) {
   ilu_grid = std::max(1, std::min(bpf, 4)) * num_sms;
   cudaError_t es = cudaStreamSynchronize(s);
   if (es != cudaSuccess) return ctx.cuda_fail(es, "batch upload");
+  if ((rc0 = build_local(ctx, plan))) return rc0;
   return set_tiles(ctx);
+}
+
+bool Batch::use_local(const Ctx &ctx) const { return local.tasks + streams.tasks > 0 && ctx.task_sweep < 0; }
+
+// Device tables of the batch's local tasks (the plan's lists, and per member the slot of every row,
+// the columns in task numbers and the forward result by slot) and of its streams.
+int Batch::build_local(Ctx &ctx, const SweepPlan &plan) {
+  nrest = plan.nrest;
+  own_kernel = plan.own_kernel;
+  cudaError_t e;
+  cudaStream_t s = ctx.stream;
+#define ALLOC(ptr, bytes)                                   \
+  ptr = arena.alloc(size_t(bytes), e);                      \
+  if (!ptr) return ctx.cuda_fail(e, "cudaMalloc batch " #ptr);
+#define TABLE(dst, vec)                                                                                                       \
+  ALLOC(dst, std::max<size_t>(sizeof(vec[0]) * vec.size(), 16));                                                                \
+  if (!vec.empty() && (e = cudaMemcpyAsync(dst, vec.data(), sizeof(vec[0]) * vec.size(), cudaMemcpyHostToDevice, s)) != cudaSuccess) \
+    return ctx.cuda_fail(e, "upload batch " #dst);
+  const LocalPlan &L = plan.local;
+  std::vector<LocSys> ls(sys.size(), LocSys{});
+  if (plan.nlocal) {
+    local.tasks = plan.nlocal;
+    local.consumers = L.consumers; local.ring = L.ring; local.stage = L.stage;
+    TABLE(local.d_tasks, L.tasks);
+    TABLE(local.d_chunks, L.chunks);
+    TABLE(local.d_copies, L.copies);
+    TABLE(local.d_heads, L.heads);
+    for (size_t k = 0; k < sys.size(); ++k) {
+      if (plan.fmap[k].empty()) continue;
+      const System *S = sys[k];
+      void *yslot, *fslot, *lcol, *ucol;
+      ALLOC(yslot, sizeof(double) * size_t(S->n + kVecPad));
+      ALLOC(fslot, sizeof(int32_t) * size_t(S->n + kVecPad));
+      ALLOC(lcol, sizeof(int32_t) * size_t(std::max<int64_t>(S->padL, 1)));
+      ALLOC(ucol, sizeof(int32_t) * size_t(std::max<int64_t>(S->padU, 1)));
+      // the maps pass through the forward result's buffer, which no sweep has written yet
+      int32_t *f = (int32_t *)yslot, *b = f + S->n;
+      if ((e = cudaMemsetAsync(fslot, 0, sizeof(int32_t) * size_t(S->n + kVecPad), s)) != cudaSuccess ||
+          (e = cudaMemcpyAsync(f, plan.fmap[k].data(), sizeof(int32_t) * size_t(S->n), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
+          (e = cudaMemcpyAsync(b, plan.bmap[k].data(), sizeof(int32_t) * size_t(S->n), cudaMemcpyHostToDevice, s)) != cudaSuccess)
+        return ctx.cuda_fail(e, "upload task numbers");
+      int rc = vk_slots(S->n, S->d_dpos, (int32_t *)fslot, s);
+      if (!rc) rc = vk_map_columns(S->n, S->padL, S->d_lcol, f, (int32_t *)lcol, s);
+      if (!rc) rc = vk_map_columns(S->n, S->padU, S->d_ucol, b, (int32_t *)ucol, s);
+      if (rc) return ctx.cuda_fail(cudaError_t(rc), "local sweep tables");
+      if ((e = cudaMemsetAsync(yslot, 0, sizeof(double) * size_t(S->n + kVecPad), s)) != cudaSuccess) return ctx.cuda_fail(e, "memset");
+      ls[k] = LocSys{(const int32_t *)lcol, (const int32_t *)ucol, (const int32_t *)fslot, (double *)yslot};
+    }
+    TABLE(local.d_sys, ls);
+  }
+  std::vector<StreamTask> st;
+  for (size_t t = size_t(plan.nrest + plan.nlocal); t < plan.tasks.size(); ++t) {
+    const int32_t k = plan.tasks[t].sys;
+    const System *S = sys[size_t(k)];
+    const StreamPlan &Q = S->stream;
+    StreamTask T{};
+    T.sys = k; T.nwarp = Q.nwarp; T.nchunk = int32_t(Q.chunks.size()); T.nfwd = Q.nfwd; T.ring = Q.ring; T.stage = Q.stage;
+    T.keep[0] = Q.keep[0]; T.keep[1] = Q.keep[1];
+    std::memcpy(T.width, Q.width, sizeof(T.width));
+    T.chunks = S->d_stream; T.heads = S->d_stream_heads; T.ent = S->d_stream_ent; T.row = S->d_stream_row; T.olds = S->d_stream_olds;
+    T.yslot = S->d_yslot;
+    st.push_back(T);
+    streams.nwarp = std::max(streams.nwarp, Q.nwarp);
+    streams.smem = std::max(streams.smem, int(local_smem_bytes(Q.ring, Q.stage)));
+  }
+  streams.tasks = int(st.size());
+  if (streams.tasks) { TABLE(streams.d_tasks, st); }
+#undef ALLOC
+#undef TABLE
+  if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return ctx.cuda_fail(e, "local sweep tables");
+  return VSHE_OK;
 }
 
 // Row tiles (whole SELL slices: multiples of 32 rows) that never straddle two systems; the tile
@@ -1624,6 +2117,7 @@ int Batch::factor(Ctx &ctx) {
       vk_split_factor_f32(S->nnzF, S->n, S->d_lu64, S->d_fmap, S->d_pdiag, S->d_dpos, (float *)S->d_lval, (float *)S->d_uval, (float *)S->d_udinv, s);
     else
       vk_split_factor_f64(S->nnzF, S->n, S->d_lu64, S->d_fmap, S->d_pdiag, S->d_dpos, (double *)S->d_lval, (double *)S->d_uval, (double *)S->d_udinv, s);
+    if (S->d_stream && (rc = S->fill_stream(ctx, false))) return rc;
   }
   return check_err(ctx, "ilu0 factorisation");
 }
@@ -1635,28 +2129,51 @@ int Batch::factor(Ctx &ctx) {
 // batch on its own factors (one forward + backward apply, CUDA events), before the first
 // iteration; the choice does not change any result (each slice is computed the same way by
 // whichever warp, in either kind).
-// The task sweep launched: task_kernel 0 = one CTA per task with the factor slices staged
+// The task sweep launched: the batch's local tasks with k_trsv_local and its streams with
+// k_trsv_stream (unless vshe_set_task_sweep names a kernel), the others with task_kernel: 0 = one CTA per task with the factor slices staged
 // through shared memory (k_trsv_task), K > 0 = one thread-block cluster of K CTAs per task
 // (k_trsv_cluster).
 int Batch::launch_tasks(Ctx &ctx, int which) {
   cudaStream_t s = ctx.stream;
-  if (task_kernel == 0)
-    return mixed ? vk_trsv_task_f32(ntasks, d_sysdev, d_state, d_active, d_tasks, d_chunks, d_sdesc, which, d_bar, d_err, s)
-                 : vk_trsv_task_f64(ntasks, d_sysdev, d_state, d_active, d_tasks, d_chunks, d_sdesc, which, d_bar, d_err, s);
-  return mixed ? vk_trsv_cluster_f32(ntasks, task_kernel, d_sysdev, d_state, d_active, d_ctasks, d_clv, which, s)
-               : vk_trsv_cluster_f64(ntasks, task_kernel, d_sysdev, d_state, d_active, d_ctasks, d_clv, which, s);
+  int count = ntasks;
+  if (use_local(ctx)) {
+    int rc = 0;
+    if (streams.tasks)
+      rc = vk_trsv_stream(mixed ? 1 : 0, streams.tasks, streams.nwarp, streams.smem, d_sysdev, d_state, d_active, streams.d_tasks, which, d_bar,
+                          d_err, s);
+    if (!rc && local.tasks)
+      rc = vk_trsv_local(mixed ? 1 : 0, local.tasks, local.consumers, local.ring, local.stage, d_sysdev, d_state, d_active, local.d_sys,
+                         local.d_tasks, local.d_chunks, local.d_copies, local.d_heads, which, d_bar, d_err, s);
+    if (rc) return rc;
+    count = nrest;
+  }
+  return count ? launch_task_kernel(ctx, count, which) : 0;
 }
 
-// Autotuner of the task sweep: one apply of each candidate (staged single CTA; clusters of 2, 4
+// the first `count` tasks with k_trsv_task or k_trsv_cluster
+int Batch::launch_task_kernel(Ctx &ctx, int count, int which) {
+  cudaStream_t s = ctx.stream;
+  if (task_kernel == 0)
+    return mixed ? vk_trsv_task_f32(count, d_sysdev, d_state, d_active, d_tasks, d_chunks, d_sdesc, which, d_bar, d_err, s)
+                 : vk_trsv_task_f64(count, d_sysdev, d_state, d_active, d_tasks, d_chunks, d_sdesc, which, d_bar, d_err, s);
+  return mixed ? vk_trsv_cluster_f32(count, task_kernel, d_sysdev, d_state, d_active, d_ctasks, d_clv, which, s)
+               : vk_trsv_cluster_f64(count, task_kernel, d_sysdev, d_state, d_active, d_ctasks, d_clv, which, s);
+}
+
+// Autotuner of the task sweep of the tasks that are not local: one apply of each candidate (staged single CTA; clusters of 2, 4
 // and 8 CTAs) timed on the batch's own factors with CUDA events, once per batch before its first
 // iteration; the fastest is kept.  Every candidate computes every row the same way, so the
 // choice changes no result.
 int Batch::autotune_tasks(Ctx &ctx) {
+  if (use_local(ctx) != local_captured) {  // vshe_set_task_sweep since the chunk was captured
+    local_captured = use_local(ctx);
+    if (chunk_exec) { cudaGraphExecDestroy(chunk_exec); chunk_exec = nullptr; }
+  }
   if (ctx.task_sweep >= 0 && task_kernel != ctx.task_sweep) {
     task_kernel = ctx.task_sweep;
     if (chunk_exec) { cudaGraphExecDestroy(chunk_exec); chunk_exec = nullptr; }
   }
-  if (ctx.task_sweep >= 0 || tasks_tuned || !has_pc || ntasks == 0) return VSHE_OK;
+  if (ctx.task_sweep >= 0 || tasks_tuned || !has_pc || ntasks == 0 || nrest == 0) return VSHE_OK;
   tasks_tuned = true;
   {
     auto it = ctx.task_choice.find(tune_key_tasks);
@@ -1676,9 +2193,9 @@ int Batch::autotune_tasks(Ctx &ctx) {
   task_tune_ms.clear();
   for (int k : {0, 2, 4, 8}) {
     task_kernel = k;
-    int rc = launch_tasks(ctx, 0);  // warm-up
+    int rc = launch_task_kernel(ctx, nrest, 0);  // warm-up
     cudaEventRecord(a, s);
-    for (int r = 0; r < 3; ++r) rc |= launch_tasks(ctx, 0);
+    for (int r = 0; r < 3; ++r) rc |= launch_task_kernel(ctx, nrest, 0);
     cudaEventRecord(b, s);
     cudaError_t e = cudaEventSynchronize(b);
     if (rc || e != cudaSuccess) { cudaEventDestroy(a); cudaEventDestroy(b); return ctx.cuda_fail(e != cudaSuccess ? e : cudaError_t(rc), "autotune task sweeps"); }
@@ -2032,7 +2549,7 @@ int Batch::solve(Ctx &ctx, std::vector<vshe_solve_stats> &stats) {
     st.levels_U = S->nlevU;
     st.bytes_device = int64_t(S->arena.total);
     const int tk = task_kind.empty() ? 0 : task_kind[size_t(k)];
-    st.sweep_ctas = !has_pc ? 0 : tk ? (task_kernel > 0 ? task_kernel : 1) : trsv_grid;
+    st.sweep_ctas = !has_pc ? 0 : tk ? (task_kernel > 0 && !(use_local(ctx) && own_kernel[size_t(k)]) ? task_kernel : 1) : trsv_grid;
     st.sweep_mode = !has_pc ? 0
                     : tk == 1 ? VSHE_TRSV_PER_SYSTEM
                     : tk == 2 ? VSHE_TRSV_PER_BLOCK
@@ -2486,6 +3003,87 @@ int vshe_layout_sweep_plan(int64_t n, int64_t nnz, const int64_t *rp, const int3
       const int32_t v[4] = {d.soff, d.width, d.r0, d.nr};
       std::copy(v, v + 4, sdesc + 4 * k);
     }
+  return VSHE_OK;
+}
+
+int vshe_layout_local_plan(int64_t n, int64_t nnz, const int64_t *rp, const int32_t *ci, const double *val, const vshe_solve_opts *opts,
+                           int32_t num_sms, int64_t *counts, int32_t *tasks, int32_t *chunks, int64_t *copies, uint8_t *heads, int32_t *fmap,
+                           int32_t *bmap) {
+  if (!counts) return VSHE_E_INVALID_ARGUMENT;
+  Layout L;
+  int rc = layout_for(n, nnz, rp, ci, val, opts, L);
+  if (rc) return rc;
+  System S;
+  S.n = n;
+  S.nnz = nnz;
+  if (opts) S.opts = *opts; else vshe_default_opts(&S.opts);
+  S.adopt_layout(L);
+  SweepPlan P;
+  plan_sweep_tasks(std::vector<System *>{&S}, S.mixed, S.has_pc, num_sms > 0 ? num_sms : 148, P);
+  const LocalPlan &Q = P.local;
+  const int64_t c[9] = {int64_t(Q.tasks.size()), int64_t(Q.chunks.size()), int64_t(Q.copies.size()), int64_t(Q.heads.size()),
+                        Q.consumers, Q.ring, Q.stage, P.nrest, 0};
+  std::copy(c, c + 9, counts);
+  if (tasks)
+    for (size_t t = 0; t < Q.tasks.size(); ++t) {
+      const LocTask &d = Q.tasks[t];
+      const int32_t v[8] = {d.sys, d.c0, d.nfwd, d.nchunk, d.nlevF, d.m, d.ring, 0};
+      std::copy(v, v + 8, tasks + 8 * t);
+    }
+  if (chunks)
+    for (size_t k = 0; k < Q.chunks.size(); ++k) {
+      const LocChunk &d = Q.chunks[k];
+      const int32_t v[5] = {d.rec0, d.nrec, d.nlate, d.bytes, d.late_bytes};
+      std::copy(v, v + 5, chunks + 5 * k);
+    }
+  if (copies)
+    for (size_t k = 0; k < Q.copies.size(); ++k) {
+      const LocCopy &d = Q.copies[k];
+      const int64_t v[4] = {d.src, d.dst, d.what >> 24, d.what & 0xffffff};
+      std::copy(v, v + 4, copies + 4 * k);
+    }
+  if (heads) std::copy(Q.heads.begin(), Q.heads.end(), heads);
+  for (int64_t i = 0; i < n && !P.fmap.empty() && !P.fmap[0].empty(); ++i) {
+    if (fmap) fmap[i] = P.fmap[0][size_t(i)];
+    if (bmap) bmap[i] = P.bmap[0][size_t(i)];
+  }
+  return VSHE_OK;
+}
+
+int vshe_layout_stream_plan(int64_t n, int64_t nnz, const int64_t *rp, const int32_t *ci, const double *val, const vshe_solve_opts *opts,
+                            int64_t *counts, int64_t *chunks, int32_t *steps, int64_t *recs, int64_t *patch, int32_t *olds, uint8_t *widths) {
+  if (!counts) return VSHE_E_INVALID_ARGUMENT;
+  Layout L;
+  int rc = layout_for(n, nnz, rp, ci, val, opts, L);
+  if (rc) return rc;
+  System S;
+  S.n = n;
+  S.nnz = nnz;
+  if (opts) S.opts = *opts; else vshe_default_opts(&S.opts);
+  S.adopt_layout(L);
+  StreamPlan P;
+  if (sweep_kind(S, S.mixed) == 1) plan_stream(S, L, P);
+  const int64_t c[12] = {P.ok ? 1 : 0, P.nwarp, P.ring, P.stage, P.nfwd, P.keep[0], P.keep[1], int64_t(P.chunks.size()),
+                         int64_t(P.heads.size() / sizeof(StreamStep)), int64_t(P.recs.size()), int64_t(P.patch.size() / 2),
+                         P.ok ? local_smem_bytes(P.ring, P.stage) : 0};
+  std::copy(c, c + 12, counts);
+  if (!P.ok) return VSHE_OK;
+  if (chunks)
+    for (size_t k = 0; k < P.chunks.size(); ++k) {
+      const StreamChunk &d = P.chunks[k];
+      const int64_t v[11] = {d.head, d.ent, d.row, d.head_bytes, d.ent_bytes, d.row_bytes, d.op0, d.nop, d.nstep, d.old0, d.nold};
+      std::copy(v, v + 11, chunks + 11 * k);
+    }
+  if (steps) std::memcpy(steps, P.heads.data(), P.heads.size());
+  if (recs)
+    for (size_t k = 0; k < P.recs.size(); ++k) {
+      const StreamRec &d = P.recs[k];
+      const int64_t v[5] = {d.ent, d.row, d.slice, d.width, d.lower};
+      std::copy(v, v + 5, recs + 5 * k);
+    }
+  if (patch) std::copy(P.patch.begin(), P.patch.end(), patch);
+  if (olds) std::copy(P.olds.begin(), P.olds.end(), olds);
+  if (widths) std::copy(&P.width[0][0], &P.width[0][0] + 32, widths);
   return VSHE_OK;
 }
 

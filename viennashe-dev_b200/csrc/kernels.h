@@ -60,6 +60,22 @@ void vk_precond_copy(int ntiles, const void *sys, const void *st, const VkTiles 
 VK_DECL_P(float, f32)
 VK_DECL_P(double, f64)
 
+// the apply of block tasks whose solved values fit shared memory (trsv_local.cu), the slot of every
+// row, and columns in task numbers
+int vk_trsv_local(int mixed, int ntasks, int consumers, int ring, int stage_bytes, const void *sys, const void *st, const int32_t *act,
+                  const void *lsys, const void *tasks, const void *chunks, const void *copies, const void *heads, int which, const unsigned *bar,
+                  int32_t *err, cudaStream_t s);
+int vk_slots(int64_t n, const int64_t *dpos, int32_t *fslot, cudaStream_t s);
+int vk_map_columns(int64_t n, int64_t count, const int32_t *col, const int32_t *map, int32_t *out, cudaStream_t s);
+
+// the apply of whole systems with many short levels (trsv_stream.cu), and the fill of a system's stream
+// (sysdev: the host's SysDev): all = 1 its tables, 0 the factor's values; patch: (entry, shared-memory
+// offset) of the entries older than the ring
+int vk_trsv_stream(int mixed, int ntasks, int nwarp, int smem, const void *sys, const void *st, const int32_t *act, const void *tasks, int which,
+                   const unsigned *bar, int32_t *err, cudaStream_t s);
+int vk_stream_fill(int mixed, const void *sysdev, int nrec, const void *recs, const int64_t *dpos, int ring, int npatch, const int64_t *patch,
+                   int all, void *ent, void *row, cudaStream_t s);
+
 // y = A x on a SELL-32 matrix (solver order)
 void vk_spmv_plain(int grid, int64_t n, const int64_t *aoff, const int32_t *acol, const double *aval, const double *x, double *y, cudaStream_t s);
 // out[q] = in[perm[q]] (gather = 1) or out[perm[q]] = in[q] (gather = 0)

@@ -138,6 +138,59 @@ inline constexpr int64_t task_chunk_bytes(int64_t ns, int64_t nslot, int64_t r0,
   return 16 * ns + (4 + vbytes) * nslot + (r1 - r0) * (lower ? 8 : 4 + vbytes);
 }
 
+// Local sweep tasks (k_trsv_local): block tasks whose solved values fit shared memory.  A task
+// numbers its rows 0 .. m-1 in the order its forward sweep solves them, its backward slots likewise in
+// the order of the backward sweep; its factor columns are given in these numbers (LocSys), and the CTA
+// keeps value i at entry i of a shared-memory array of `ring` >= m entries.
+//
+// A chunk is a run of the task's slices, across levels, that fits one shared-memory stage:
+//   LocHead, int32 wptr[consumers + 1], SliceLoc[slices] (16-byte aligned; sorted by the
+//   consumer warp that sums them, wptr = each warp's range), factor columns, factor values, then
+//   per row operand, aligned runs of rows or slots one after the other: A = the input vector's rows
+//   (forward) or the forward result by slot (backward), FP64; B = the row's backward slot
+//   (forward) or the slot's row (backward); C = inverse diagonals (backward).
+// LocCopy lists the copies that fill it: bytes from (array `kind`) + src to stage offset dst.
+// Copies of the forward result come last (nlate) and wait for the forward sweep.
+struct LocTask {
+  int32_t sys, c0, nfwd, nchunk;  // chunks [c0, c0 + nchunk), the first nfwd forward
+  int32_t nlevF, nbar;            // forward levels; level barriers of the whole task
+  int32_t m, ring;
+};
+struct LocChunk {
+  int32_t rec0, nrec, nlate;   // copies [rec0, rec0 + nrec), the last nlate after the forward sweep
+  int32_t bytes, late_bytes;   // of the first nrec - nlate copies, and of the others
+};
+struct LocCopy {
+  int64_t src;   // byte offset in the array of that kind
+  int32_t dst;   // byte offset in the stage
+  int32_t what;  // kind << 24 | bytes
+};
+enum LocKind { kLocHead = 0, kLocLCol, kLocLVal, kLocIn, kLocFSlot, kLocUCol, kLocUVal, kLocYSlot, kLocURow, kLocUDinv, kLocKinds };
+struct LocHead {
+  int32_t offA, offB, offC;  // stage offsets of the row operands
+  int32_t offD;              // stage offset of the slice descriptors
+  int32_t pass;              // level barriers to have passed before the next chunk is waited for
+  int32_t pad[3];
+};
+struct SliceLoc {
+  int32_t col, val;    // stage offsets of the slice's columns and values
+  int32_t op;          // index of its first row in the chunk's operand runs
+  int32_t wnr;         // width << 6 | rows
+  int32_t loc0, lev;   // number of its first row; level barriers to pass before its gathers
+  int32_t pad[2];
+};
+// Per system of a batch: columns in task numbers (padding: kLocPad), backward slot of every row, and
+// the forward result by backward slot.
+constexpr int32_t kLocPad = 0x7fffffff;
+struct LocSys {
+  const int32_t *lcol, *ucol, *fslot;
+  double *yslot;
+};
+constexpr int kLocStages = 3;
+constexpr int kLocNarrow = 15, kLocWide = 31;  // most consumer warps with 128 and with 64 registers a thread
+constexpr int64_t kLocSmemMax = 229632;        // shared memory a CTA may ask for, less the kernel's static part
+inline constexpr int64_t local_smem_bytes(int64_t ring, int64_t stage_bytes) { return 8 * ring + 128 + kLocStages * stage_bytes; }
+
 // Cluster sweep tasks (k_trsv_cluster): the same units as TaskDev, walked by one thread-block
 // cluster each, level by level, with the slices of level k of the forward (backward) sweep in
 // [lv[offL + 2k], lv[offL + 2k + 1]) ([lv[offU + 2k], ...)).
@@ -145,6 +198,68 @@ struct ClusterTask {
   int32_t sys, nlevL, nlevU, pad;
   int64_t offL, offU;
 };
+
+// Streams (k_trsv_stream): a whole system laid out for one CTA that walks many short levels.  The
+// levels are cut into steps of at most `nwarp` slices of one level, one slice per warp; every warp
+// takes part in every step (with an empty slice where it has none) and in the barrier before each.
+// Row i of a sweep (forward: the solver row, backward: the slot) keeps its value at i mod `ring` of a
+// shared-memory ring.  An entry whose column is older than the ring when its level ends (number below
+// level end - ring) is read from its chunk's stage, where the producer gathers such values from global
+// memory: the rows of three consecutive chunks fit the ring, so they are solved and written by all
+// warps when the chunk is fetched.
+//
+// Device arrays, filled by k_stream_fill (the values anew after every factorisation) from the SELL slices:
+//   entries: for slice record r, w entries of 32 lanes: StreamEnt (shared-memory byte offset of the
+//            solved value it multiplies; factor value)
+//   rows:    for slice record r, 32 StreamRow (where the lane's value goes, inverse diagonal)
+// A chunk is a run of whole steps (an even number) that fits one shared-memory stage: step descriptors
+// (StreamStep, nwarp per step, two steps more than it has), entries, rows (the first slice of both is
+// the chunk's empty one), values older than the ring, and the sweep's operand rows (the input, or the
+// forward result by slot).
+template <typename P> struct StreamEnt;
+template <> struct __attribute__((aligned(8))) StreamEnt<float> { int32_t at; float v; };
+template <> struct __attribute__((aligned(16))) StreamEnt<double> { int32_t at, pad; double v; };
+struct __attribute__((aligned(16))) StreamRow {
+  int32_t pos;   // ring position in bytes
+  int32_t dst;   // forward: the row's slot; backward: the slot's row; -1: no row
+  double dinv;
+};
+struct StreamStep {
+  int32_t ent;    // stage offset of the slice's entries
+  int32_t row;    // of its rows
+  int32_t op;     // of its first operand
+  int32_t width;  // entries stored
+};
+struct StreamChunk {
+  int64_t head, ent, row;                    // byte offsets in the system's arrays
+  int32_t head_bytes, ent_bytes, row_bytes;
+  int32_t op0, nop;                          // operand rows [op0, op0 + nop), multiples of 4
+  int32_t nstep;                             // steps, each after a barrier
+  int32_t old0, nold;                        // values older than the ring: numbers olds[old0, old0 + nold)
+  int32_t pad;
+};
+// one slice of the stream, for k_stream_fill
+struct StreamRec {
+  int64_t ent, row;        // byte offsets in the system's arrays
+  int32_t slice, width;    // SELL slice (negative: empty); entries stored (>= the slice's)
+  int32_t lower, pad;      // 1: forward
+};
+struct StreamTask {
+  int32_t sys, nwarp, nchunk, nfwd, ring, stage;
+  int32_t keep[2];           // forward, backward: values are read after they left the ring
+  uint8_t width[2][16];      // per sweep and warp: the entries its slices are stored with (above kStreamW: own widths)
+  const StreamChunk *chunks;
+  const unsigned char *heads, *ent, *row;
+  const int32_t *olds;
+  double *yslot;           // forward result by slot
+};
+constexpr int kStreamW = 8;         // slices up to this wide are stored at their chunk's width
+constexpr int kStreamWarps = 15;    // most warps of a stream
+// the kernel's variant for a warp whose widest slice is w: entries stored per slice (kStreamW + 1: at
+// least kStreamW, wider slices keep their width)
+inline constexpr int stream_width(int w) { return w <= 1 ? 1 : w <= 6 ? w : w <= kStreamW ? kStreamW : kStreamW + 1; }
+constexpr int64_t kStreamRing = 8192;         // most values a ring holds
+
 
 // FP64 residual view of one system (solver order): r = b - A x.
 struct RefDev {

@@ -135,6 +135,59 @@ def sweep_plan(rp, ci, values=None, num_sms=148, **kw):
     return {"kind": int(cnt[3]), "tasks": tasks, "chunks": chunks, "sdesc": sdesc}
 
 
+def local_plan(rp, ci, values=None, num_sms=148, **kw):
+    """vshe_layout_local_plan: the local tasks of one system's sweep plan (host only) -> dict of the
+    launch shape and the tables "tasks" (t, 8), "chunks" (c, 5), "copies" (k, 4), "heads" (bytes),
+    "fmap", "bmap" (n)."""
+    L = lib()
+    rp = np.ascontiguousarray(rp, np.int64)
+    ci = np.ascontiguousarray(ci, np.int32)
+    n = len(rp) - 1
+    o, keep = make_opts(**kw)
+    vals = None if values is None else np.ascontiguousarray(values, np.float64)
+    L.vshe_layout_local_plan.argtypes = [C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(SolveOptsC),
+                                         C.c_int32] + [C.c_void_p] * 7
+    cnt = np.zeros(9, np.int64)
+    args = (n, int(rp[-1]), rp.ctypes.data, ci.ctypes.data, None if vals is None else vals.ctypes.data, C.byref(o), int(num_sms))
+    rc = L.vshe_layout_local_plan(*args, cnt.ctypes.data, *[None] * 6)
+    if rc:
+        raise VsheError(rc, "vshe_layout_local_plan")
+    t = {"tasks": np.zeros((int(cnt[0]), 8), np.int32), "chunks": np.zeros((int(cnt[1]), 5), np.int32),
+         "copies": np.zeros((int(cnt[2]), 4), np.int64), "heads": np.zeros(int(cnt[3]), np.uint8),
+         "fmap": np.zeros(n, np.int32), "bmap": np.zeros(n, np.int32)}
+    rc = L.vshe_layout_local_plan(*args, cnt.ctypes.data, *[t[k].ctypes.data for k in ("tasks", "chunks", "copies", "heads", "fmap", "bmap")])
+    if rc:
+        raise VsheError(rc, "vshe_layout_local_plan")
+    t.update(zip(("consumers", "ring", "stage", "rest"), (int(v) for v in cnt[4:])))
+    return t
+
+
+def stream_plan(rp, ci, values=None, **kw):
+    """vshe_layout_stream_plan: the stream of one system (host only) -> dict of its shape and the tables
+    "chunks" (c, 11), "steps" (k, 4), "recs" (r, 5), "patch" (p, 2), "olds", "widths" (2, 16), or None
+    if it has none."""
+    L = lib()
+    rp = np.ascontiguousarray(rp, np.int64)
+    ci = np.ascontiguousarray(ci, np.int32)
+    o, keep = make_opts(**kw)
+    vals = None if values is None else np.ascontiguousarray(values, np.float64)
+    L.vshe_layout_stream_plan.argtypes = [C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(SolveOptsC)] + [C.c_void_p] * 7
+    cnt = np.zeros(12, np.int64)
+    args = (len(rp) - 1, int(rp[-1]), rp.ctypes.data, ci.ctypes.data, None if vals is None else vals.ctypes.data, C.byref(o))
+    rc = L.vshe_layout_stream_plan(*args, cnt.ctypes.data, *[None] * 6)
+    if rc:
+        raise VsheError(rc, "vshe_layout_stream_plan")
+    if not cnt[0]:
+        return None
+    t = {"chunks": np.zeros((int(cnt[7]), 11), np.int64), "steps": np.zeros((int(cnt[8]), 4), np.int32), "recs": np.zeros((int(cnt[9]), 5), np.int64),
+         "patch": np.zeros((int(cnt[10]), 2), np.int64), "olds": np.zeros(int(cnt[10] + cnt[7]), np.int32), "widths": np.zeros((2, 16), np.uint8)}
+    rc = L.vshe_layout_stream_plan(*args, cnt.ctypes.data, *[t[k].ctypes.data for k in ("chunks", "steps", "recs", "patch", "olds", "widths")])
+    if rc:
+        raise VsheError(rc, "vshe_layout_stream_plan")
+    t.update(zip(("nwarp", "ring", "stage", "nfwd"), (int(v) for v in cnt[1:5])), keep=(int(cnt[5]), int(cnt[6])), smem=int(cnt[11]))
+    return t
+
+
 def kernel_launches():
     """This library's own kernel launches in the process so far."""
     return int(lib().vshe_kernel_launches())
