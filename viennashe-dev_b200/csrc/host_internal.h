@@ -194,6 +194,9 @@ struct Batch {
   int32_t nlevL = 0, nlevU = 0;   // merged levels of the grid-wide sweeps
   int32_t nlevF = 0;              // merged levels of the factorisation (all members)
   int trsv_grid = 148, ilu_grid = 148, num_sms = 148;
+  // members factorised by one thread-block cluster each (d_chain: their indexes); the others share levF
+  int nchain = 0, chain_cluster = 1;
+  int32_t *d_chain = nullptr;
   // sweep tasks (k_trsv_task: one CTA per preconditioner block or per system, TaskDev / ChunkDev
   // tables, ordered by decreasing work); members not swept as tasks share the merged level
   // schedule of the grid-wide sweep (grid_group)

@@ -1769,7 +1769,7 @@ int Batch::build(Ctx &ctx, const std::vector<System *> &members) {
   }
   task_kind.assign(on_task.begin(), on_task.end());
   std::vector<int64_t> cptrL, cptrU, fptr;
-  std::vector<int32_t> csL, cqL, csU, cqU, fsys, frow;
+  std::vector<int32_t> csL, cqL, csU, cqU, fsys, frow, chain;
   auto slices = [&](bool lower, std::vector<int64_t> &cptr, std::vector<int32_t> &cs, std::vector<int32_t> &cq, int32_t &nl) {
     nl = 0;
     for (int k = 0; k < nsys; ++k)
@@ -1793,14 +1793,20 @@ int Batch::build(Ctx &ctx, const std::vector<System *> &members) {
     slices(false, cptrU, csU, cqU, nlevU);
     // factorisation: merged level l = the forward-level-l rows of every member (all members,
     // whichever sweep they use)
+    // Members swept as one task whose levels hold up to 1024 rows on average are factorised by a
+    // cluster of CTAs each (k_ilu_cluster): the levels are short, so that the barrier after each sets the
+    // time, and it is cheaper the fewer CTAs it joins.
+    std::vector<char> on_chain(size_t(nsys), 0);
+    for (int k = 0; k < nsys; ++k) on_chain[size_t(k)] = on_task[size_t(k)] == 1 && sys[size_t(k)]->n <= 1024 * int64_t(sys[size_t(k)]->nlevL);
     nlevF = 0;
-    for (System *S : sys) nlevF = std::max(nlevF, S->nlevL);
+    for (int k = 0; k < nsys; ++k)
+      if (!on_chain[size_t(k)]) nlevF = std::max(nlevF, sys[size_t(k)]->nlevL);
     if (nsys > 1) {
       fptr.assign(1, 0);
       for (int32_t l = 0; l < nlevF; ++l) {
         for (int k = 0; k < nsys; ++k) {
           const System *S = sys[size_t(k)];
-          if (l + 1 >= int32_t(S->lvr.size())) continue;
+          if (on_chain[size_t(k)] || l + 1 >= int32_t(S->lvr.size())) continue;
           for (int64_t q = S->lvr[size_t(l)]; q < S->lvr[size_t(l) + 1]; ++q) {
             fsys.push_back(k);
             frow.push_back(int32_t(q));
@@ -1809,6 +1815,17 @@ int Batch::build(Ctx &ctx, const std::vector<System *> &members) {
         fptr.push_back(int64_t(fsys.size()));
       }
     }
+    // Its CTAs hold the rows of an average level and half as many again (ILUT rows take 128 threads, the
+    // others 8 lanes, of 512 threads).
+    double need = 0;
+    for (int k = 0; k < nsys; ++k) {
+      if (!on_chain[size_t(k)]) continue;
+      const System *S = sys[size_t(k)];
+      chain.push_back(k);
+      need = std::max(need, 1.5 * double(S->n) / std::max(S->nlevL, 1) / (S->opts.precond == VSHE_PRECOND_ILUT ? 4.0 : 64.0));
+    }
+    nchain = int(chain.size());
+    chain_cluster = need <= 1 ? 1 : need <= 2 ? 2 : need <= 4 ? 4 : 8;
   }
   cudaError_t e;
 #define ALLOC(ptr, type, count)                                              \
@@ -1844,6 +1861,7 @@ int Batch::build(Ctx &ctx, const std::vector<System *> &members) {
     ALLOC(d_cqL, int32_t, std::max<size_t>(cqL.size(), 1));
     ALLOC(d_csU, int32_t, std::max<size_t>(csU.size(), 1));
     ALLOC(d_cqU, int32_t, std::max<size_t>(cqU.size(), 1));
+    if (nchain) { ALLOC(d_chain, int32_t, nchain); }
     if (nsys > 1) {
       ALLOC(d_fptr, int64_t, fptr.size());
       ALLOC(d_fsys, int32_t, std::max<size_t>(fsys.size(), 1));
@@ -1861,7 +1879,7 @@ int Batch::build(Ctx &ctx, const std::vector<System *> &members) {
     // the final / replacement residual is written into the Krylov r
     RefDev r{S->n, S->d_aoff, S->d_acol, S->d_aval, S->d_bp, (const double *)S->kv[0], (double *)S->kv[1]};
     std::memcpy(rd.data() + vk_refdev_size() * size_t(k), &r, sizeof(r));
-    FactDev f{S->n, S->d_prp, S->d_pci, S->d_lu64, S->d_pdiag, S->d_blk, 0, 0, 0.0};
+    FactDev f{S->n, S->d_prp, S->d_pci, S->d_lu64, S->d_pdiag, S->d_blk, 0, 0, 0.0, S->d_lvr, S->nlevL};
     if (S->opts.precond == VSHE_PRECOND_ILUT) {
       f.ilut = 1;
       f.pkeep = S->opts.ilut_entries > 0 ? S->opts.ilut_entries : 60;
@@ -1894,6 +1912,7 @@ int Batch::build(Ctx &ctx, const std::vector<System *> &members) {
       H2D(d_csU, csU.data(), sizeof(int32_t) * csU.size());
       H2D(d_cqU, cqU.data(), sizeof(int32_t) * cqU.size());
     }
+    if (nchain) { H2D(d_chain, chain.data(), sizeof(int32_t) * chain.size()); }
     if (nsys > 1) {
       H2D(d_fptr, fptr.data(), sizeof(int64_t) * fptr.size());
       if (!fsys.empty()) {
@@ -2110,7 +2129,9 @@ int Batch::factor(Ctx &ctx) {
   if (rs) return rs;
   cudaStream_t s = ctx.stream;
   const int mode = (sys[0]->opts.trsv_mode == VSHE_TRSV_PER_LEVEL) ? 2 : 1;
-  int rc = vk_ilu0(mode, mode == 1 ? ilu_grid : std::max(1, num_sms * 8), d_factdev, &levF, d_bar, d_err, s);
+  int rc = 0;
+  if (nchain) rc = vk_ilu_cluster(nchain, chain_cluster, d_factdev, d_chain, d_err, s);
+  if (!rc && nchain < nsys) rc = vk_ilu0(mode, mode == 1 ? ilu_grid : std::max(1, num_sms * 8), d_factdev, &levF, d_bar, d_err, s);
   if (rc) return ctx.cuda_fail(cudaError_t(rc), "ilu0 launch");
   for (System *S : sys) {
     if (mixed)
@@ -2130,9 +2151,9 @@ int Batch::factor(Ctx &ctx) {
 // iteration; the choice does not change any result (each slice is computed the same way by
 // whichever warp, in either kind).
 // The task sweep launched: the batch's local tasks with k_trsv_local and its streams with
-// k_trsv_stream (unless vshe_set_task_sweep names a kernel), the others with task_kernel: 0 = one CTA per task with the factor slices staged
-// through shared memory (k_trsv_task), K > 0 = one thread-block cluster of K CTAs per task
-// (k_trsv_cluster).
+// k_trsv_stream (unless vshe_set_task_sweep names a kernel), the others with task_kernel: 0 = one
+// CTA per task with the factor slices staged through shared memory (k_trsv_task), K > 0 = one
+// thread-block cluster of K CTAs per task (k_trsv_cluster).
 int Batch::launch_tasks(Ctx &ctx, int which) {
   cudaStream_t s = ctx.stream;
   int count = ntasks;
@@ -2160,8 +2181,8 @@ int Batch::launch_task_kernel(Ctx &ctx, int count, int which) {
                : vk_trsv_cluster_f64(count, task_kernel, d_sysdev, d_state, d_active, d_ctasks, d_clv, which, s);
 }
 
-// Autotuner of the task sweep of the tasks that are not local: one apply of each candidate (staged single CTA; clusters of 2, 4
-// and 8 CTAs) timed on the batch's own factors with CUDA events, once per batch before its first
+// Autotuner of the task sweep of the tasks without a kernel of their own: one apply of each
+// candidate (staged single CTA; clusters of 2, 4 and 8 CTAs) timed on the batch's own factors with CUDA events, once per batch before its first
 // iteration; the fastest is kept.  Every candidate computes every row the same way, so the
 // choice changes no result.
 int Batch::autotune_tasks(Ctx &ctx) {

@@ -82,6 +82,8 @@ void vk_spmv_plain(int grid, int64_t n, const int64_t *aoff, const int32_t *acol
 void vk_permute(int64_t n, const int32_t *perm, const double *in, double *out, int gather, cudaStream_t s);
 
 int vk_ilu0(int mode, int grid, const void *fs, const VkLevels *lv, unsigned *bar, int32_t *err, cudaStream_t s);
+// the members (indexes into fs) factorised by one cluster of csize CTAs each
+int vk_ilu_cluster(int nmembers, int csize, const void *fs, const int32_t *members, int32_t *err, cudaStream_t s);
 int vk_ilu0_occupancy(int *blocks_per_sm);
 // out[k] = av[amap[k]] (0 where amap[k] < 0)
 void vk_gather_values(int64_t nnz, const int64_t *amap, const double *av, double *out, cudaStream_t s);

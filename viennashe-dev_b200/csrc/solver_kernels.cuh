@@ -94,6 +94,9 @@ struct FactDev {
   // the pkeep largest entries of the row's L part and of its U part are kept
   int32_t ilut, pkeep;
   double tau;
+  // forward levels: rows [lvr[k], lvr[k + 1])
+  const int64_t *lvr;
+  int32_t nlev;
 };
 
 // Sweep tasks.  A task is one independent unit of the incomplete-LU apply that one CTA walks

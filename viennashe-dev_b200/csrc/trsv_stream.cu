@@ -257,7 +257,13 @@ __global__ void __launch_bounds__(32 * (kStreamWarps + 1), 1)
   // the forward result is complete: hand this thread's part to the bulk copies
   fence_async_proxy();
   __syncwarp();
-  if (ok && lane == 0) mbar_arrive(&fwd);
+  if (!ok) {
+    // (no further chunk wait: the phase parities tell nothing once a phase has been given up)
+    for (int q = T.nfwd; q < T.nchunk; ++q)
+      for (int b = 0; b < T.chunks[q].nstep; ++b) consumers_sync(k.nwarp * 32);
+    return;
+  }
+  if (lane == 0) mbar_arrive(&fwd);
   k.dst = which == 0 ? S.ph : S.sh;
   k.g0 = T.nfwd;
   k.g1 = T.nchunk;
