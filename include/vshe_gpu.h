@@ -267,23 +267,21 @@ int vshe_layout_sweep_plan(int64_t n, int64_t nnz, const int64_t *row_ptr, const
                            int64_t *chunks, int32_t *sdesc);
 
 /* The local part of the same plan: the block tasks whose solved values fit shared memory
- * (k_trsv_local), for tests of the stage and ring bounds.
- * - counts[0..8]: tasks, chunks, copies, bytes of chunk heads, consumer warps, ring entries, bytes of
- *   a stage, the tasks of the plan that are neither local nor streams, 0.
- * - tasks[8 t ..]: system, first chunk, forward chunks, chunks, forward levels, rows, ring, 0.
- * - chunks[5 c ..]: first copy, copies, of them after the forward sweep, bytes of the former, bytes of
- *   the latter.
- * - copies[4 k ..]: source offset (bytes), stage offset, array (0 heads, 1 / 2 forward columns /
- *   values, 3 input, 4 slot of every row, 5 / 6 backward columns / values, 7 forward result by slot,
- *   8 row of every slot, 9 inverse diagonals), bytes.
- * - heads: per chunk int32 offsets of the operands A, B, C and of the slice descriptors, barriers to
- *   pass, 3 unused, the warps' descriptor ranges (consumers + 1), and the descriptors (int32 column
- *   offset, value offset, operand index, width * 64 + rows, first row's number, level, 2 unused).
- * - fmap / bmap[n]: the number of every solver row in its task's forward and backward sweep.
+ * (k_trsv_local), for tests of its bounds.
+ * - counts[0..9]: tasks, warps, records, bytes of all records, warps per task, shared-memory values,
+ *   slots per warp, bytes of a slot, the tasks of the plan that are neither local nor streams, runs.
+ * - tasks[6 t ..]: system, forward levels, levels, rows, first warp, first run.
+ * - runs[2 k ..]: first row of a forward level and its number.
+ * - warps[5 w ..]: byte offset of its first chunk, its chunks, sizes of the first three.
+ * - recs[9 r ..]: byte offset, SELL slice, its first column, columns, 1 forward, number of its first row
+ *   (forward), barriers before its gathers, groups of four columns, rows (0: not the slice's last
+ *   record; + 64 in a backward slice).  With a negative slice, a chunk: its records and the
+ *   size of the chunk slots - 1 further on, in places 5 and 6.
+ * - num[n]: the number of every solver row in its task.
  * Call once with NULL arrays for the counts.  Host only. */
 int vshe_layout_local_plan(int64_t n, int64_t nnz, const int64_t *row_ptr, const int32_t *col, const double *val,
-                           const vshe_solve_opts *opts, int32_t num_sms, int64_t *counts, int32_t *tasks, int32_t *chunks,
-                           int64_t *copies, uint8_t *heads, int32_t *fmap, int32_t *bmap);
+                           const vshe_solve_opts *opts, int32_t num_sms, int64_t *counts, int32_t *tasks, int32_t *runs,
+                           int64_t *warps, int64_t *recs, int32_t *num);
 /* The stream of a system swept as one task (k_trsv_stream), for tests of its bounds.
  * - counts[0..11]: 1 if the system has one, warps, ring entries, bytes of a stage, forward chunks, 1 if
  *   forward / backward values are read after they left the ring, chunks, step descriptors, slices,

@@ -63,7 +63,9 @@ def test_stream_equals_task(precision, n, offsets):
 @pytest.mark.parametrize("sizes, offsets", [
     ([1] * 40, [-1, 1]), ([32] * 40, [-1, 1]), ([33, 1, 7, 64, 500] * 9, [-3, -1, 1, 3]),
     ([3000] * 170, [-60, -1, 1, 60]),                                   # more blocks than tasks
-    ([16384, 16385, 200, 16000], [-128, -1, 1, 128]),                   # around what fits shared memory
+    ([16384, 16385, 200, 16000], [-128, -1, 1, 128]),                   # long levels: k_trsv_task
+    # below and above what fits shared memory
+    ([19800, 20000, 23500, 23700, 16000], [-700, -251, -250, -126, -125, -3, -2, -1, 1, 2, 3, 125, 126, 250, 251, 700]),
 ])
 def test_local_equals_task(precision, sizes, offsets):
     blocks = np.concatenate([[0], np.cumsum(sizes)])

@@ -9,8 +9,8 @@ bit for bit with the level by level sweep of the same SELL slices:
 * a value a row reads from the ring is the one it names, of an earlier level, and no row of the
   reader's own level overwrites it; one read from global memory (by streams) is at
   least three steps old;
-* block tasks: a warp's slices come in level order, and every chunk's barrier count lets the warps
-  still in it reach their levels;
+* block tasks: a warp's chunks follow each other, and each is copied whole into a slot that its reader
+  has left;
 * streams: every warp has a slice (the chunk's empty one where it has none) in every step, and the
   descriptors reach two steps past the end;
 * over all tasks every row is solved once forward and once backward."""
@@ -66,6 +66,14 @@ BLOCKS = {
     "bar_blocks_fp64": (lambda: _system(lambda: D.config2(40, 10, 48, 3)), BLK, "fp64", 2),
     "bar_blocks_L1": (lambda: _system(lambda: D.config2(37, 9, 55, 1)), dict(BLK, fill_level=0), "mixed", 2),
 }
+def _many_blocks(size=310, count=170):
+    """More blocks than CTAs: tasks of two blocks."""
+    n = size * count
+    rp, ci, v, _ = _far(n, 61)
+    return rp, ci, v, np.arange(0, n + 1, size)
+
+
+BLOCKS["tasks_of_two_blocks"] = (_many_blocks, dict(BLK, trsv="per_block"), "mixed", 2)
 STREAMS = {
     "diode_mixed": (lambda: _system(D.config1), NAT, "mixed", 1),
     "diode_fp64": (lambda: _system(D.config1), NAT, "fp64", 1),
@@ -233,86 +241,116 @@ def test_stream_runs_like_the_level_sweep(name):
     assert np.array_equal(out, z_ref)
 
 
+@pytest.mark.parametrize("num_sms", [148, 20])
 @pytest.mark.parametrize("name", sorted(BLOCKS))
-def test_local_plan_runs_like_the_level_sweep(name):
+def test_local_plan_runs_like_the_level_sweep(name, num_sms):
     rp, ci, vals, kw, lay, vt, lval, uval, udinv, x, slot, (y_ref, z_ref) = _make(BLOCKS[name])
-    P = gpu.local_plan(rp, ci, vals, **kw)
-    n, ring, C = lay["n"], P["ring"], P["consumers"]
-    assert len(P["tasks"]) > 0 and P["rest"] == 0
-    assert C in (3, 7, 15, 31) and ring & (ring - 1) == 0
-    assert 8 * ring + 128 + 3 * P["stage"] + 256 <= SMEM
-    assert (8 * ring + 128) % 128 == 0 and P["stage"] % 128 == 0, "copies into the stages are 16-byte aligned"
-    fm, bm = np.append(P["fmap"], PAD), np.append(P["bmap"], PAD)
-    arrays = {0: P["heads"], 1: fm[lay["lcol"]].astype(np.int32), 2: lval, 3: x, 4: slot, 5: bm[lay["ucol"]].astype(np.int32), 6: uval,
-              7: np.full(n + 8, np.nan), 8: np.concatenate([lay["urow"], np.zeros(8, np.int32)]), 9: udinv}
-    vb = vt().itemsize
+    P = gpu.local_plan(rp, ci, vals, num_sms=num_sms, **kw)
+    n, ring, nw, slots, sb = lay["n"], P["ring"], P["nwarp"], P["slots"], P["slot_bytes"]
+    vb = np.dtype(vt).itemsize
+    assert 1 <= nw <= 15 and 2 <= slots <= 3 and ring % 16 == 0 and ring < 1 << 16 and sb % 16 == 0
+    assert 8 * ring + 128 + nw * slots * sb + 1024 <= SMEM
+    assert len(P["tasks"]) and P["rest"] == 0 and len(P["warps"]) == nw * len(P["tasks"])
+    # the chunks and records as k_local_fill writes them, by offset; they follow each other without a gap
+    recs, chunks, end, left, cols = {}, {}, 0, 0, 8
+    seen = {True: np.zeros(len(lay["lcol"]) // 32, int), False: np.zeros(len(lay["ucol"]) // 32, int)}
+    rows = {True: np.zeros(n, int), False: np.zeros(n, int)}
+    for off, j, u0, ncol, lower, loc0, lev, groups, nr in P["recs"].tolist():
+        assert off == end and off % 16 == 0
+        if j < 0:
+            assert left == 0 and loc0 > 0
+            head, left, end = off, loc0, off + 16
+            chunks[head] = [16, lev, []]
+            continue
+        lower, back, nr = bool(lower), nr >= 64, nr % 64
+        size = 16 + 128 * groups * (2 + vb) + (32 * (2 + vb) if back else 0)
+        end, left = off + size, left - 1
+        chunks[head][0] += size
+        chunks[head][2].append(off)
+        assert size % 16 == 0 and chunks[head][0] <= sb
+        so, col, val, r0 = (lay["loff"], lay["lcol"], lval, lay["lrow0"]) if lower else (lay["uoff"], lay["ucol"], uval, lay["uslot0"])
+        w = int(so[j + 1] - so[j]) // 32
+        last = u0 + ncol == w
+        assert 0 <= ncol <= cols and u0 % cols == 0 and (nr > 0) == last and (last or ncol == cols)
+        assert back == (last and not lower) and 4 * groups - ncol in (0, 1, 2, 3)
+        a, b = so[j] + 32 * u0, so[j] + 32 * (u0 + ncol)
+        seen[lower][a // 32:b // 32] += 1
+        q = np.arange(r0[j], r0[j + 1])
+        if last:
+            assert nr == len(q)
+            rows[lower][q] += 1
+        c = col[a:b].reshape(ncol, 32).astype(np.int64)
+        num = np.where(c < n, P["num"][np.minimum(c, n - 1)], ring)
+        assert np.all(num[c < n] < ring)
+        loc = P["num"][q if lower else lay["urow"][q]]
+        assert not lower or np.array_equal(loc, loc0 + np.arange(len(q)))
+        recs[off] = (loc, nr, lev, lower, q, num, val[a:b].reshape(ncol, 32), np.where(c < n, c, -1))
+    assert end == P["bytes"] and left == 0
+    assert all(np.all(k == 1) for k in seen.values()) and all(np.all(k == 1) for k in rows.values())
     out = np.full(n, np.nan)
-    fwd_seen, bwd_seen = np.zeros(n, int), np.zeros(n, int)
-    for sys_, c0, nfwd, nchunk, nlevF, m, tring, _ in P["tasks"].tolist():
-        assert tring == ring and m <= ring
-        win, tlev = np.full(ring, np.nan), np.full(ring, -1)
-        passed = 0
-        writes = []  # (level, number, value): applied when their level closes
-        for g in range(c0, c0 + nchunk):
-            lower = g - c0 < nfwd
-            if g - c0 == nfwd:
-                win[:], tlev[:] = np.nan, -1  # nothing of the forward sweep is read again
-            rec0, nrec, nlate, nbytes, late = P["chunks"][g].tolist()
-            stage, used = np.zeros(P["stage"], np.uint8), np.zeros(P["stage"], bool)
-            tot = [0, 0]
-            for k in range(rec0, rec0 + nrec):
-                src, dst, arr, size = P["copies"][k].tolist()
-                b = arrays[arr].view(np.uint8)
-                assert src % 16 == 0 and dst % 16 == 0 and size % 16 == 0 and size > 0
-                assert src + size <= len(b) and dst + size <= P["stage"] and not used[dst:dst + size].any()
-                is_late = k >= rec0 + nrec - nlate
-                assert is_late == (arr == 7)
-                stage[dst:dst + size], used[dst:dst + size] = b[src:src + size], True
-                tot[is_late] += size
-            assert tot == [nbytes, late]
-            i32 = stage.view(np.int32)
-            offA, offB, offC, offD, npass = i32[:5].tolist()
-            wptr = i32[8:8 + C + 1]
-            ns = int(wptr[C])
-            desc = i32[offD // 4:offD // 4 + 8 * ns].reshape(ns, 8)
-            assert wptr[0] == 0 and np.all(np.diff(wptr) >= 0) and offD + 32 * ns <= offA
-            for w in range(C):
-                assert np.all(np.diff(desc[wptr[w]:wptr[w + 1], 5]) >= 0), "a warp's slices come in level order"
-            lmax = int(desc[:, 5].max())
-            assert npass == (nlevF if g - c0 == nfwd - 1 else lmax)
-            for d in desc[np.argsort(desc[:, 4], kind="stable")]:
-                col, val, op, wnr, loc0, lev = d[:6].tolist()
-                width, nr = wnr >> 6, wnr & 63
-                if lev > passed:  # the level barrier: what earlier levels wrote is visible
-                    for l_, num, value in writes:
-                        win[num], tlev[num] = value, l_
-                    writes, passed = [], lev
-                c = i32[col // 4:col // 4 + 32 * width].reshape(width, 32)[:, :nr]
-                a = stage[val:val + 32 * width * vb].view(vt).reshape(width, 32)[:, :nr].astype(float)
-                s = np.zeros(nr)
-                for k in range(width):
-                    q = c[k]
-                    near = q < m
-                    assert np.all(q[near] < loc0) and np.all(tlev[q[near]] < lev) and np.all(tlev[q[near]] >= 0)
-                    xv = np.zeros(nr)
-                    xv[near] = win[q[near]]
-                    s = s + a[k] * xv
-                num = np.arange(loc0, loc0 + nr)
-                assert loc0 + nr <= m
-                base = stage[offA:].view(np.float64)[op:op + nr]
-                dst = stage[offB:].view(np.int32)[op:op + nr]
-                assert used[offA + 8 * op:offA + 8 * (op + nr)].all() and used[offB + 4 * op:offB + 4 * (op + nr)].all()
-                if lower:
-                    r = base - s
-                    arrays[7][dst] = r
-                    fwd_seen[dst] += 1
-                else:
-                    r = (base - s) * stage[offC:].view(vt)[op:op + nr].astype(float)
-                    out[dst] = r
-                    bwd_seen[dst] += 1
-                writes += [(lev, t, value) for t, value in zip(num.tolist(), r.tolist())]
-            if g - c0 == nfwd - 1:
-                writes, passed = [], nlevF
-    assert np.all(fwd_seen == 1) and np.all(bwd_seen == 1)
-    assert np.array_equal(arrays[7][slot[:n]], y_ref)
+    for sys, nlevF, nlev, m, w0, run0 in P["tasks"].tolist():
+        assert 0 < m <= ring and 0 < nlevF < nlev
+        W = P["warps"][w0:w0 + nw].tolist()
+        # entry i: value, row, forward result (1) or backward (2)
+        win, who, kind = np.full(ring + 1, np.nan), np.full(ring + 1, -1), np.zeros(ring + 1, int)
+        win[ring] = 0.0
+        runs = P["runs"][run0:run0 + nlevF]
+        for (row, num), stop in zip(runs, np.append(runs[1:, 1], m)):
+            who[num:stop] = np.arange(row, row + stop - num)
+            win[num:stop] = x[who[num:stop]]
+        assert np.all(who[:m] >= 0) and np.array_equal(P["num"][who[:m]], np.arange(m))
+        nxt, held, todo, done = [w[0] for w in W], [[None] * slots for _ in W], [[] for _ in W], [0] * nw
+        acc = [np.zeros(32) for _ in W]
+
+        def issue(k, to, size):
+            assert held[k][to] is None and size == chunks[nxt[k]][0], "a whole chunk into a free slot"
+            held[k][to] = nxt[k]
+            nxt[k] += size
+
+        for k, w in enumerate(W):
+            for i in range(min(slots - 1, w[1])):
+                issue(k, i, w[2 + i])
+        # between two barriers the warps run in any order: what they write is not read by others before the
+        # next; the results are read after the last
+        for passed in range(nlev):
+            if passed == nlevF:
+                assert np.all(kind[:m] == 1), "the forward sweep ends before this barrier"
+            writes = []
+            for k in range(nw):
+                while True:
+                    if not todo[k]:
+                        # the chunk before this one is read to its end: its slot is free
+                        if done[k]:
+                            held[k][(done[k] - 1) % slots] = None
+                        if done[k] == W[k][1]:
+                            break
+                        size, ahead, todo[k] = chunks[held[k][done[k] % slots]]
+                        todo[k] = list(todo[k])
+                        if ahead:
+                            issue(k, (done[k] + slots - 1) % slots, ahead)
+                        done[k] += 1
+                    loc, nr, lev, lower, q, num, v, named = recs[todo[k][0]]
+                    if lev != passed:
+                        assert lev > passed
+                        break
+                    todo[k].pop(0)
+                    assert lower == (passed < nlevF)
+                    used = named >= 0
+                    assert np.array_equal(who[num[used]], named[used]), "the value is the one the row names, of this task"
+                    assert np.all(kind[num[used]] == (1 if lower else 2)), "and of an earlier level of this sweep"
+                    for u in range(v.shape[0]):
+                        acc[k] = acc[k] + v[u] * win[num[u]]
+                    if nr == 0:
+                        continue
+                    assert np.all(kind[loc] == (0 if lower else 1))
+                    z = win[loc] - acc[k][:nr] if lower else (win[loc] - acc[k][:nr]) * udinv[q]
+                    acc[k] = np.zeros(32)
+                    writes += list(zip(loc.tolist(), z, [1 if lower else 2] * nr))
+            assert len({p_ for p_, _, _ in writes}) == len(writes)
+            for p_, v_, f_ in writes:
+                win[p_], kind[p_] = v_, f_
+            if passed == nlevF - 1:
+                assert np.array_equal(win[:m], y_ref[who[:m]])
+        assert done == [w[1] for w in W] and not any(todo) and np.all(kind[:m] == 2)
+        out[who[:m]] = win[:m]
     assert np.array_equal(out, z_ref)

@@ -158,13 +158,16 @@ struct System {
 // Sweep plan of a batch: per member 0 (grid-wide sweep), 1 (one task for the system) or 2 (tasks of
 // preconditioner blocks); the tasks, the chunks of their levels, the chunks' slice descriptors,
 // and the level slice ranges of the cluster sweeps.
-// Local tasks of a batch (LocTask, k_trsv_local): the tables the kernel reads and its launch shape.
+// Local tasks of a batch (k_trsv_local): the tables the kernel reads, every member's records (member k:
+// recs [rec0[k], rec0[k + 1])), the records' size and the launch shape.
 struct LocalPlan {
   std::vector<LocTask> tasks;
-  std::vector<LocChunk> chunks;
-  std::vector<LocCopy> copies;
-  std::vector<unsigned char> heads;
-  int consumers = 0, ring = 0, stage = 0;
+  std::vector<LocRun> runs;
+  std::vector<LocWarp> warps;
+  std::vector<LocRec> recs;
+  std::vector<int64_t> rec0;
+  int64_t bytes = 0;
+  int nwarp = 0, ring = 0, slots = 0, slot_bytes = 0;
 };
 struct SweepPlan {
   std::vector<char> on_task;
@@ -180,9 +183,8 @@ struct SweepPlan {
   int nrest = 0, nlocal = 0;
   LocalPlan local;
   std::vector<char> own_kernel;  // 1: no task of this member is among the first nrest
-  // per member with local block tasks: the task numbers of its rows in the forward and of their slots
-  // in the backward sweep, by solver row
-  std::vector<std::vector<int32_t>> fmap, bmap;
+  // per member with local block tasks: the task numbers of its rows, by solver row
+  std::vector<std::vector<int32_t>> lnum;
 };
 void plan_sweep_tasks(const std::vector<System *> &sys, bool mixed, bool has_pc, int64_t num_sms, SweepPlan &plan);
 
@@ -212,8 +214,10 @@ struct Batch {
   // streams (trsv_stream.cu) unless vshe_set_task_sweep names a kernel for all
   int nrest = 0;
   struct LocalTables {
-    int tasks = 0, consumers = 0, ring = 0, stage = 0;
-    void *d_tasks = nullptr, *d_chunks = nullptr, *d_copies = nullptr, *d_heads = nullptr, *d_sys = nullptr;
+    int tasks = 0, nwarp = 0, ring = 0, slots = 0, slot_bytes = 0;
+    void *d_tasks = nullptr, *d_runs = nullptr, *d_warps = nullptr, *d_recs = nullptr, *d_buf = nullptr;
+    std::vector<int64_t> rec0;
+    bool filled = false;  // the records hold the members' present factors
   } local;
   struct StreamTables {
     int tasks = 0, nwarp = 0, smem = 0;
@@ -221,6 +225,7 @@ struct Batch {
   } streams;
   std::vector<char> own_kernel;
   int build_local(Ctx &ctx, const SweepPlan &plan);
+  int fill_local(Ctx &ctx);
   bool use_local(const Ctx &ctx) const;
   bool local_captured = false;  // use_local when the chunk's graph was captured
   int launch_tasks(Ctx &ctx, int which);

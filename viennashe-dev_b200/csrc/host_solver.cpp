@@ -1196,151 +1196,99 @@ int sweep_kind(const System &S, bool mixed) {
   return 0;
 }
 
-// Bytes of a chunk head with its warp ranges and slice descriptors.
-static int64_t local_head_bytes(int consumers, int64_t ns) {
-  return ((int64_t(sizeof(LocHead)) + 4 * (consumers + 1) + 15) & ~int64_t(15)) + int64_t(sizeof(SliceLoc)) * ns;
-}
-
-// Appends the chunks of the sweep plan's task t to a local plan (LocTask in solver_kernels.cuh).
-static void add_local_task(const std::vector<System *> &sys, int vb, SweepPlan &P, size_t t, int64_t m) {
+// Records of the sweep plan's task t (LocHead in solver_kernels.cuh), and the task numbers of its rows.
+static void add_local_task(const std::vector<System *> &sys, int vb, SweepPlan &P, size_t t, int64_t m, int nwarp) {
   LocalPlan &L = P.local;
   const ClusterTask &c = P.ctasks[t];
   const System *S = sys[size_t(c.sys)];
-  std::vector<int32_t> &fm = P.fmap[size_t(c.sys)], &bm = P.bmap[size_t(c.sys)];
-  if (fm.empty()) { fm.assign(size_t(S->n), kLocPad); bm.assign(size_t(S->n), kLocPad); }
-  const int C = L.consumers;
-  LocTask T{c.sys, int32_t(L.chunks.size()), 0, 0, c.nlevL, std::max(c.nlevL, c.nlevL + c.nlevU - 1), int32_t(m), L.ring};
+  std::vector<int32_t> &num = P.lnum[size_t(c.sys)];
+  if (num.empty()) num.assign(size_t(S->n), kLocPad);
+  const LocTask T{c.sys, c.nlevL, c.nlevL + c.nlevU, int32_t(m), int32_t(L.warps.size()), int32_t(L.runs.size()), {0, 0}};
+  struct Piece { int64_t slice, bytes; int32_t u0, ncol, lower; LocHead head; };
+  std::vector<std::vector<Piece>> seq((size_t)nwarp);  // per warp
+  std::vector<int64_t> total((size_t)nwarp, 0), load((size_t)nwarp);
+  std::vector<std::pair<int64_t, int64_t>> order;  // width, slice
   for (int pass = 0; pass < 2; ++pass) {
     const bool lower = pass == 0;
     const std::vector<int64_t> &off = lower ? S->loff_h : S->uoff_h, &rs = lower ? S->lrow0_h : S->uslot0_h;
     const int64_t *lv = P.clv.data() + (lower ? c.offL : c.offU);
-    const int32_t nlev = lower ? c.nlevL : c.nlevU, lev0 = lower ? 0 : c.nlevL;
-    // operand bytes per row or slot: FP64 operand, int32 target, inverse diagonal (backward)
-    const int64_t row_bytes = lower ? 12 : 12 + vb;
-    // the chunk being filled: its slices with their warps, operand runs (aligned row ranges), slot runs
-    struct Item { SliceLoc d; int warp; };
-    std::vector<Item> items;
-    std::vector<std::pair<int64_t, int64_t>> runs, slots;
-    int64_t nslot = 0, nop = 0, last_end = -1, loc = 0;
-    int32_t lmax = 0;
-    auto flush = [&](bool last) {
-      if (items.empty()) return;
-      const int64_t ns = int64_t(items.size()), hb = local_head_bytes(C, ns), offcol = hb, offval = offcol + 4 * nslot, offA = offval + vb * nslot,
-                    offB = offA + 8 * nop, offC = offB + 4 * nop;
-      std::stable_sort(items.begin(), items.end(), [](const Item &x, const Item &y) { return x.warp < y.warp; });
-      const size_t h0 = L.heads.size();
-      L.heads.resize(h0 + size_t(hb), 0);
-      const LocHead H{int32_t(offA), int32_t(offB), int32_t(offC), int32_t(hb - int64_t(sizeof(SliceLoc)) * ns),
-                      last && lower ? c.nlevL : lmax, {0, 0, 0}};
-      std::memcpy(L.heads.data() + h0, &H, sizeof(H));
-      std::vector<int32_t> wptr((size_t)C + 1, 0);
-      for (const Item &it : items) wptr[size_t(it.warp) + 1]++;
-      for (int w = 0; w < C; ++w) wptr[size_t(w) + 1] += wptr[size_t(w)];
-      std::memcpy(L.heads.data() + h0 + sizeof(H), wptr.data(), 4 * wptr.size());
-      for (int64_t k = 0; k < ns; ++k) {
-        SliceLoc d = items[size_t(k)].d;
-        d.val = int32_t(offval + int64_t(d.col) * vb);
-        d.col = int32_t(offcol + int64_t(d.col) * 4);
-        std::memcpy(L.heads.data() + h0 + size_t(H.offD) + size_t(k) * sizeof(SliceLoc), &d, sizeof(d));
-      }
-      LocChunk ch{int32_t(L.copies.size()), 0, 0, 0, 0};
-      auto copy = [&](int kind, int64_t src, int64_t dst, int64_t bytes) {
-        if (bytes <= 0) return;
-        L.copies.push_back({src, int32_t(dst), int32_t(kind << 24 | int(bytes))});
-        ch.bytes += int32_t(bytes);
-      };
-      copy(kLocHead, int64_t(h0), 0, hb);
-      int64_t at = 0;
-      for (auto &r : slots) {
-        copy(lower ? kLocLCol : kLocUCol, 4 * r.first, offcol + 4 * at, 4 * (r.second - r.first));
-        copy(lower ? kLocLVal : kLocUVal, vb * r.first, offval + vb * at, vb * (r.second - r.first));
-        at += r.second - r.first;
-      }
-      at = 0;
-      for (auto &r : runs) {
-        const int64_t k = r.second - r.first;
-        if (lower) {
-          copy(kLocIn, 8 * r.first, offA + 8 * at, 8 * k);
-          copy(kLocFSlot, 4 * r.first, offB + 4 * at, 4 * k);
-        } else {
-          copy(kLocURow, 4 * r.first, offB + 4 * at, 4 * k);
-          copy(kLocUDinv, vb * r.first, offC + vb * at, vb * k);
+    int64_t loc = 0;
+    for (int32_t k = 0; k < (lower ? c.nlevL : c.nlevU); ++k) {
+      const int64_t a = lv[2 * k], b = lv[2 * k + 1], first = rs[size_t(a)];
+      order.clear();
+      for (int64_t j = a; j < b; ++j) order.push_back({(off[size_t(j)] - off[size_t(j) + 1]) >> 5, j});
+      std::sort(order.begin(), order.end());
+      std::fill(load.begin(), load.end(), 0);
+      for (auto &o : order) {
+        const int64_t j = o.second, r0 = rs[size_t(j)], r1 = rs[size_t(j) + 1], w = -o.first;
+        size_t to = 0;
+        for (size_t q = 1; q < size_t(nwarp); ++q)
+          if (load[q] < load[to] || (load[q] == load[to] && total[q] < total[to])) to = q;
+        load[to] += w + 8;
+        total[to] += w + 8;
+        for (int64_t u = 0;; u += kLocCols) {
+          const bool last = u + kLocCols >= w, back = last && !lower;
+          const int64_t nc = std::min<int64_t>(w - u, kLocCols), groups = (nc + 3) / 4;
+          seq[to].push_back(Piece{j, local_rec_bytes(groups, back, vb), int32_t(u), int32_t(nc), lower ? 1 : 0,
+                                  LocHead{int32_t(loc + r0 - first), (lower ? 0 : c.nlevL) + k, int32_t(groups),
+                                          last ? int32_t(r1 - r0) + (back ? kLocBack : 0) : 0}});
+          if (last) break;
         }
-        at += k;
       }
-      if (!lower) {
-        const int32_t early = ch.bytes;
-        const size_t n0 = L.copies.size();
-        at = 0;
-        for (auto &r : runs) { copy(kLocYSlot, 8 * r.first, offA + 8 * at, 8 * (r.second - r.first)); at += r.second - r.first; }
-        ch.nlate = int32_t(L.copies.size() - n0);
-        ch.late_bytes = ch.bytes - early;
-        ch.bytes = early;
-      }
-      ch.nrec = int32_t(L.copies.size()) - ch.rec0;
-      L.chunks.push_back(ch);
-      items.clear(); runs.clear(); slots.clear();
-      nslot = nop = 0;
-      last_end = -1;
-    };
-    for (int32_t k = 0; k < nlev; ++k) {
-      const int64_t a = lv[2 * k], b = lv[2 * k + 1];
-      for (int64_t j = a; j < b; ++j) {
-        const int64_t r0 = rs[size_t(j)], r1 = rs[size_t(j) + 1], w = off[size_t(j) + 1] - off[size_t(j)];
-        for (int tries = 0; tries < 2; ++tries) {
-          // operand entries this slice adds: its rows extend the last run, or start a new aligned one
-          const bool extend = last_end == r0;
-          const int64_t e1 = (r1 + 3) & ~int64_t(3), e0 = extend ? runs.back().second : (r0 & ~int64_t(3));
-          const int64_t add = std::max<int64_t>(e1 - e0, 0);
-          if (tries == 0 && local_head_bytes(C, int64_t(items.size()) + 1) + (4 + vb) * (nslot + w) + row_bytes * (nop + add) > L.stage) {
-            flush(false);
-            continue;
-          }
-          if (extend) runs.back().second = std::max(runs.back().second, e1);
-          else runs.push_back({e0, e1});
-          const int64_t op = nop + add - (runs.back().second - r0);
-          if (!slots.empty() && slots.back().second == off[size_t(j)]) slots.back().second += w;
-          else if (w > 0) slots.push_back({off[size_t(j)], off[size_t(j)] + w});
-          const SliceLoc d{int32_t(nslot), 0, int32_t(op), int32_t((w >> 5) << 6 | (r1 - r0)), int32_t(loc), lev0 + k, {0, 0}};
-          items.push_back({d, int((j - a) % C)});
-          nslot += w;
-          nop += add;
-          last_end = r1;
-          lmax = lev0 + k;
-          break;
-        }
-        for (int64_t r = r0; r < r1; ++r) {
-          if (lower) fm[size_t(r)] = int32_t(loc + r - r0);
-          else bm[size_t(S->urow_h[size_t(r)])] = int32_t(loc + r - r0);
-        }
-        loc += r1 - r0;
+      if (lower) {
+        L.runs.push_back(LocRun{int32_t(first), int32_t(loc)});
+        for (int64_t r = first; r < rs[size_t(b)]; ++r) num[size_t(r)] = int32_t(loc + r - first);
+        loc += rs[size_t(b)] - first;
       }
     }
-    flush(true);
-    if (lower) T.nfwd = int32_t(L.chunks.size()) - T.c0;
   }
-  T.nchunk = int32_t(L.chunks.size()) - T.c0;
+  for (int w = 0; w < nwarp; ++w) {
+    const std::vector<Piece> &q = seq[size_t(w)];
+    std::vector<std::pair<size_t, int64_t>> chunks;  // records up to, bytes
+    for (size_t i = 0; i < q.size(); ++i) {
+      if (chunks.empty() || chunks.back().second + q[i].bytes > L.slot_bytes) chunks.push_back({i, int64_t(sizeof(LocChunk))});
+      chunks.back().first = i + 1;
+      chunks.back().second += q[i].bytes;
+    }
+    auto bytes = [&](size_t i) { return i < chunks.size() ? int32_t(chunks[i].second) : 0; };
+    L.warps.push_back(LocWarp{L.bytes, int32_t(chunks.size()), {bytes(0), bytes(1), bytes(2)}});
+    for (size_t h = 0, i = 0; h < chunks.size(); ++h) {
+      LocRec R{L.bytes, -1, 0, 0, 0, {}};
+      const LocChunk C{int32_t(chunks[h].first - i), bytes(h + size_t(L.slots) - 1), {0, 0}};
+      static_assert(sizeof(C) == sizeof(R.head), "");
+      std::memcpy(&R.head, &C, sizeof(C));
+      L.recs.push_back(R);
+      L.bytes += int64_t(sizeof(C));
+      for (; i < chunks[h].first; ++i) {
+        L.recs.push_back(LocRec{L.bytes, int32_t(q[i].slice), q[i].u0, q[i].ncol, q[i].lower, q[i].head});
+        L.bytes += q[i].bytes;
+      }
+    }
+  }
   L.tasks.push_back(T);
 }
 
-// Splits the tasks by kernel.  Whole systems with a stream take k_trsv_stream.  A block task whose
-// rows all fit the ring of shared memory is local (k_trsv_local); one stage size serves the batch:
-// 32 KB, or what its widest slice needs up to 64 KB, and the ring is the largest power of two
-// beside the stages (16384 values with 32 KB stages).  Larger blocks (energy slabs of large 2D
-// meshes) keep k_trsv_task: the colours of a block spread a row's neighbours over the whole slab.
+// Splits the tasks by kernel.  Whole systems with a stream take k_trsv_stream.  A block task is local
+// (k_trsv_local) if its values fit shared memory beside the slots of 12 warps, about 23,000 rows (FP64
+// factors 20,000; larger ones, energy slabs of large 2D meshes, keep k_trsv_task), and an average level has at most
+// 48 slices: beyond, k_trsv_task has enough gathers in flight, and more bandwidth (tasks of 16000 rows and
+// 125 slices a level 29 us per apply against 32, 8000 rows and 62 slices 21 against 18; of 21800 rows and 8
+// neighbours 186 against 149 with 15 warps, FP64 210 against 219 with 9).  One shape serves the batch: values for the largest local task; half
+// as many warps again as an average level has slices, since the slices' widths differ (bar 50 x 20 x
+// 60, 5 slices: 9.8 us per apply with 5 warps, 9.0 with 8, 9.1 with 10; bar 90 x 29 x 64, 14 slices:
+// 97 with 12, 87 with 15); and three slots of chunks per warp, two if they do not fit.
 static void plan_local_tasks(const std::vector<System *> &sys, bool mixed, SweepPlan &P) {
   const int vb = mixed ? 4 : 8;
   const size_t nt = P.tasks.size();
   P.nrest = int(nt);
   P.nlocal = 0;
   P.own_kernel.assign(sys.size(), 0);
-  P.fmap.assign(sys.size(), {});
-  P.bmap.assign(sys.size(), {});
+  P.lnum.assign(sys.size(), {});
   P.local = LocalPlan{};
+  LocalPlan &L = P.local;
   if (nt == 0) return;
-  struct Info { int64_t m = 0, stage = 0; double slices = 0, levels = 0; };
+  struct Info { int64_t m = 0; double slices = 0, levels = 0; };
   std::vector<Info> info(nt);
-  int64_t stage = 32768;
   for (size_t t = 0; t < nt; ++t) {
     const ClusterTask &c = P.ctasks[t];
     const System *S = sys[size_t(c.sys)];
@@ -1348,32 +1296,29 @@ static void plan_local_tasks(const std::vector<System *> &sys, bool mixed, Sweep
     Info &I = info[t];
     for (int pass = 0; pass < 2; ++pass) {
       const bool lower = pass == 0;
-      const std::vector<int64_t> &off = lower ? S->loff_h : S->uoff_h, &rs = lower ? S->lrow0_h : S->uslot0_h;
+      const std::vector<int64_t> &rs = lower ? S->lrow0_h : S->uslot0_h;
       const int64_t *lv = P.clv.data() + (lower ? c.offL : c.offU);
       for (int32_t k = 0; k < (lower ? c.nlevL : c.nlevU); ++k) {
         const int64_t a = lv[2 * k], b = lv[2 * k + 1];
-        for (int64_t j = a; j < b; ++j) {
-          const int64_t nr = rs[size_t(j) + 1] - rs[size_t(j)];
-          I.stage = std::max(I.stage, local_head_bytes(kLocWide, 1) + (4 + vb) * (off[size_t(j) + 1] - off[size_t(j)]) + (nr + 6) * (12 + vb));
-        }
         if (lower) I.m += rs[size_t(b)] - rs[size_t(a)];
         I.slices += double(b - a);
         I.levels += 1;
       }
     }
-    if (I.stage <= kTaskStageBytes) stage = std::max(stage, (I.stage + 1023) & ~int64_t(1023));
   }
-  int64_t ring = 1, need = 32;
-  while (local_smem_bytes(2 * ring, stage) <= kLocSmemMax) ring *= 2;
+  constexpr int64_t kMinWarps = 12;
+  constexpr double kMostSlices = 48;
+  const int64_t slot = int64_t(sizeof(LocChunk)) + local_rec_bytes(kLocCols / 4, true, vb);
   std::vector<char> kind(nt, 0);  // 0 neither, 1 local, 2 stream
   double slices = 0, levels = 0;
+  int64_t most = 1;
   for (size_t t = 0; t < nt; ++t) {
     const Info &I = info[t];
     const size_t k = size_t(P.ctasks[t].sys);
     if (P.on_task[k] == 1) { kind[t] = sys[k]->stream.ok ? 2 : 0; continue; }
-    if (I.stage > stage || I.m > ring) continue;
+    if (8 * ((I.m + 15) & ~int64_t(15)) + 128 + kMinWarps * 2 * slot > kLocSmemMax || I.slices > kMostSlices * I.levels) continue;
     kind[t] = 1;
-    while (need < I.m) need *= 2;
+    most = std::max(most, I.m);
     slices += I.slices;
     levels += I.levels;
   }
@@ -1389,14 +1334,32 @@ static void plan_local_tasks(const std::vector<System *> &sys, bool mixed, Sweep
   P.ctasks.swap(ct);
   std::fill(P.own_kernel.begin(), P.own_kernel.end(), 1);
   for (int t = 0; t < P.nrest; ++t) P.own_kernel[size_t(P.ctasks[size_t(t)].sys)] = 0;
-  P.local.ring = int(need);
-  P.local.stage = int(stage);
-  // a little more warps than the slices of an average level, so that a level is one slice per warp
-  // and few warps only keep the level barrier company
-  P.local.consumers = 3;
-  while (P.local.consumers < kLocWide && double(P.local.consumers) < 1.1 * slices / std::max(levels, 1.0))
-    P.local.consumers = 2 * P.local.consumers + 1;
-  for (int t = P.nrest; t < P.nrest + P.nlocal; ++t) add_local_task(sys, vb, P, size_t(t), info[order[size_t(t)]].m);
+  L.rec0.assign(sys.size() + 1, 0);
+  if (P.nlocal == 0) return;
+  L.ring = int((most + 15) & ~int64_t(15));
+  const int64_t left = kLocSmemMax - 8 * int64_t(L.ring) - 128;
+  const int64_t want = std::max<int64_t>(1, int64_t(std::ceil(1.5 * slices / std::max(levels, 1.0))));
+  L.nwarp = int(std::min(std::min<int64_t>(want, kLocWarps), left / (2 * slot)));
+  L.slots = left >= 3 * slot * L.nwarp ? 3 : 2;
+  L.slot_bytes = int(std::min<int64_t>(left / (L.slots * L.nwarp), 8192) & ~int64_t(15));
+  // the tasks of a member one after the other, so that its records are one run
+  for (size_t k = 0; k < sys.size(); ++k) {
+    for (int t = P.nrest; t < P.nrest + P.nlocal; ++t)
+      if (size_t(P.ctasks[size_t(t)].sys) == k) add_local_task(sys, vb, P, size_t(t), info[order[size_t(t)]].m, L.nwarp);
+    L.rec0[k + 1] = int64_t(L.recs.size());
+  }
+  // most work first, as the plan lists them
+  std::vector<int64_t> work(L.tasks.size());
+  for (size_t t = 0; t < L.tasks.size(); ++t) {
+    const size_t w0 = size_t(L.tasks[t].warp0), w1 = w0 + size_t(L.nwarp);
+    work[t] = (w1 < L.warps.size() ? L.warps[w1].off : L.bytes) - L.warps[w0].off;
+  }
+  std::vector<size_t> by((size_t)L.tasks.size());
+  std::iota(by.begin(), by.end(), size_t(0));
+  std::stable_sort(by.begin(), by.end(), [&](size_t x, size_t y) { return work[x] > work[y]; });
+  std::vector<LocTask> sorted;
+  for (size_t t : by) sorted.push_back(L.tasks[t]);
+  L.tasks.swap(sorted);
 }
 
 // The stream of a system swept as one task: the slices of each level dealt to nwarp warps in steps, the
@@ -1966,36 +1929,25 @@ int Batch::build_local(Ctx &ctx, const SweepPlan &plan) {
   if (!vec.empty() && (e = cudaMemcpyAsync(dst, vec.data(), sizeof(vec[0]) * vec.size(), cudaMemcpyHostToDevice, s)) != cudaSuccess) \
     return ctx.cuda_fail(e, "upload batch " #dst);
   const LocalPlan &L = plan.local;
-  std::vector<LocSys> ls(sys.size(), LocSys{});
   if (plan.nlocal) {
     local.tasks = plan.nlocal;
-    local.consumers = L.consumers; local.ring = L.ring; local.stage = L.stage;
+    local.nwarp = L.nwarp; local.ring = L.ring; local.slots = L.slots; local.slot_bytes = L.slot_bytes;
+    local.rec0 = L.rec0;
     TABLE(local.d_tasks, L.tasks);
-    TABLE(local.d_chunks, L.chunks);
-    TABLE(local.d_copies, L.copies);
-    TABLE(local.d_heads, L.heads);
+    TABLE(local.d_warps, L.warps);
+    TABLE(local.d_recs, L.recs);
+    ALLOC(local.d_buf, L.bytes);
+    TABLE(local.d_runs, L.runs);
     for (size_t k = 0; k < sys.size(); ++k) {
-      if (plan.fmap[k].empty()) continue;
-      const System *S = sys[k];
-      void *yslot, *fslot, *lcol, *ucol;
-      ALLOC(yslot, sizeof(double) * size_t(S->n + kVecPad));
-      ALLOC(fslot, sizeof(int32_t) * size_t(S->n + kVecPad));
-      ALLOC(lcol, sizeof(int32_t) * size_t(std::max<int64_t>(S->padL, 1)));
-      ALLOC(ucol, sizeof(int32_t) * size_t(std::max<int64_t>(S->padU, 1)));
-      // the maps pass through the forward result's buffer, which no sweep has written yet
-      int32_t *f = (int32_t *)yslot, *b = f + S->n;
-      if ((e = cudaMemsetAsync(fslot, 0, sizeof(int32_t) * size_t(S->n + kVecPad), s)) != cudaSuccess ||
-          (e = cudaMemcpyAsync(f, plan.fmap[k].data(), sizeof(int32_t) * size_t(S->n), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-          (e = cudaMemcpyAsync(b, plan.bmap[k].data(), sizeof(int32_t) * size_t(S->n), cudaMemcpyHostToDevice, s)) != cudaSuccess)
-        return ctx.cuda_fail(e, "upload task numbers");
-      int rc = vk_slots(S->n, S->d_dpos, (int32_t *)fslot, s);
-      if (!rc) rc = vk_map_columns(S->n, S->padL, S->d_lcol, f, (int32_t *)lcol, s);
-      if (!rc) rc = vk_map_columns(S->n, S->padU, S->d_ucol, b, (int32_t *)ucol, s);
-      if (rc) return ctx.cuda_fail(cudaError_t(rc), "local sweep tables");
-      if ((e = cudaMemsetAsync(yslot, 0, sizeof(double) * size_t(S->n + kVecPad), s)) != cudaSuccess) return ctx.cuda_fail(e, "memset");
-      ls[k] = LocSys{(const int32_t *)lcol, (const int32_t *)ucol, (const int32_t *)fslot, (double *)yslot};
+      if (plan.lnum[k].empty()) continue;
+      void *num;
+      TABLE(num, plan.lnum[k]);
+      std::vector<char> sd(vk_sysdev_size());
+      sys[k]->fill_sysdev(sd.data());
+      const int rc = vk_local_fill(mixed ? 1 : 0, sd.data(), int(L.rec0[k + 1] - L.rec0[k]), (const LocRec *)local.d_recs + L.rec0[k],
+                                   (const int32_t *)num, L.ring, 1, local.d_buf, s);
+      if (rc) return ctx.cuda_fail(cudaError_t(rc), "local sweep records");
     }
-    TABLE(local.d_sys, ls);
   }
   std::vector<StreamTask> st;
   for (size_t t = size_t(plan.nrest + plan.nlocal); t < plan.tasks.size(); ++t) {
@@ -2017,6 +1969,20 @@ int Batch::build_local(Ctx &ctx, const SweepPlan &plan) {
 #undef ALLOC
 #undef TABLE
   if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return ctx.cuda_fail(e, "local sweep tables");
+  return VSHE_OK;
+}
+
+// The members' present factors into the local tasks' records: after a factorisation, and before the
+// first sweep of a batch built on members factorised before (a served batch).
+int Batch::fill_local(Ctx &ctx) {
+  for (size_t k = 0; k < sys.size() && local.tasks; ++k) {
+    std::vector<char> sd(vk_sysdev_size());
+    sys[k]->fill_sysdev(sd.data());
+    const int rc = vk_local_fill(mixed ? 1 : 0, sd.data(), int(local.rec0[k + 1] - local.rec0[k]), (const LocRec *)local.d_recs + local.rec0[k],
+                                 nullptr, local.ring, 0, local.d_buf, ctx.stream);
+    if (rc) return ctx.cuda_fail(cudaError_t(rc), "local sweep records");
+  }
+  local.filled = true;
   return VSHE_OK;
 }
 
@@ -2140,6 +2106,7 @@ int Batch::factor(Ctx &ctx) {
       vk_split_factor_f64(S->nnzF, S->n, S->d_lu64, S->d_fmap, S->d_pdiag, S->d_dpos, (double *)S->d_lval, (double *)S->d_uval, (double *)S->d_udinv, s);
     if (S->d_stream && (rc = S->fill_stream(ctx, false))) return rc;
   }
+  if ((rc = fill_local(ctx))) return rc;
   return check_err(ctx, "ilu0 factorisation");
 }
 
@@ -2163,8 +2130,8 @@ int Batch::launch_tasks(Ctx &ctx, int which) {
       rc = vk_trsv_stream(mixed ? 1 : 0, streams.tasks, streams.nwarp, streams.smem, d_sysdev, d_state, d_active, streams.d_tasks, which, d_bar,
                           d_err, s);
     if (!rc && local.tasks)
-      rc = vk_trsv_local(mixed ? 1 : 0, local.tasks, local.consumers, local.ring, local.stage, d_sysdev, d_state, d_active, local.d_sys,
-                         local.d_tasks, local.d_chunks, local.d_copies, local.d_heads, which, d_bar, d_err, s);
+      rc = vk_trsv_local(mixed ? 1 : 0, local.tasks, local.nwarp, local.ring, local.slots, local.slot_bytes, d_sysdev, d_state,
+                         d_active, local.d_tasks, local.d_runs, local.d_warps, local.d_buf, which, d_bar, d_err, s);
     if (rc) return rc;
     count = nrest;
   }
@@ -2368,6 +2335,7 @@ int Batch::write_states(Ctx &ctx, const std::vector<char> &in) {
 // replayed; under profiling, or if the driver refuses the capture, it is launched directly.
 int Batch::run_chunk(Ctx &ctx, int every) {
   int rs = sync_spin_limit(ctx);
+  if (!rs && local.tasks && !local.filled) rs = fill_local(ctx);
   if (rs) return rs;
   cudaStream_t s = ctx.stream;
   const int mode = (sys[0]->opts.trsv_mode == VSHE_TRSV_PER_LEVEL) ? 2 : trsv_kernel;
@@ -3028,8 +2996,7 @@ int vshe_layout_sweep_plan(int64_t n, int64_t nnz, const int64_t *rp, const int3
 }
 
 int vshe_layout_local_plan(int64_t n, int64_t nnz, const int64_t *rp, const int32_t *ci, const double *val, const vshe_solve_opts *opts,
-                           int32_t num_sms, int64_t *counts, int32_t *tasks, int32_t *chunks, int64_t *copies, uint8_t *heads, int32_t *fmap,
-                           int32_t *bmap) {
+                           int32_t num_sms, int64_t *counts, int32_t *tasks, int32_t *runs, int64_t *warps, int64_t *recs, int32_t *num) {
   if (!counts) return VSHE_E_INVALID_ARGUMENT;
   Layout L;
   int rc = layout_for(n, nnz, rp, ci, val, opts, L);
@@ -3042,32 +3009,29 @@ int vshe_layout_local_plan(int64_t n, int64_t nnz, const int64_t *rp, const int3
   SweepPlan P;
   plan_sweep_tasks(std::vector<System *>{&S}, S.mixed, S.has_pc, num_sms > 0 ? num_sms : 148, P);
   const LocalPlan &Q = P.local;
-  const int64_t c[9] = {int64_t(Q.tasks.size()), int64_t(Q.chunks.size()), int64_t(Q.copies.size()), int64_t(Q.heads.size()),
-                        Q.consumers, Q.ring, Q.stage, P.nrest, 0};
-  std::copy(c, c + 9, counts);
+  const int64_t c[10] = {int64_t(Q.tasks.size()), int64_t(Q.warps.size()), int64_t(Q.recs.size()), Q.bytes, Q.nwarp, Q.ring,
+                        Q.slots, Q.slot_bytes, P.nrest, int64_t(Q.runs.size())};
+  std::copy(c, c + 10, counts);
   if (tasks)
     for (size_t t = 0; t < Q.tasks.size(); ++t) {
       const LocTask &d = Q.tasks[t];
-      const int32_t v[8] = {d.sys, d.c0, d.nfwd, d.nchunk, d.nlevF, d.m, d.ring, 0};
-      std::copy(v, v + 8, tasks + 8 * t);
+      const int32_t v[6] = {d.sys, d.nlevF, d.nlev, d.m, d.warp0, d.run0};
+      std::copy(v, v + 6, tasks + 6 * t);
     }
-  if (chunks)
-    for (size_t k = 0; k < Q.chunks.size(); ++k) {
-      const LocChunk &d = Q.chunks[k];
-      const int32_t v[5] = {d.rec0, d.nrec, d.nlate, d.bytes, d.late_bytes};
-      std::copy(v, v + 5, chunks + 5 * k);
+  for (size_t k = 0; runs && k < Q.runs.size(); ++k) { runs[2 * k] = Q.runs[k].row; runs[2 * k + 1] = Q.runs[k].num; }
+  if (warps)
+    for (size_t k = 0; k < Q.warps.size(); ++k) {
+      const LocWarp &d = Q.warps[k];
+      const int64_t v[5] = {d.off, d.nchunk, d.bytes[0], d.bytes[1], d.bytes[2]};
+      std::copy(v, v + 5, warps + 5 * k);
     }
-  if (copies)
-    for (size_t k = 0; k < Q.copies.size(); ++k) {
-      const LocCopy &d = Q.copies[k];
-      const int64_t v[4] = {d.src, d.dst, d.what >> 24, d.what & 0xffffff};
-      std::copy(v, v + 4, copies + 4 * k);
+  if (recs)
+    for (size_t k = 0; k < Q.recs.size(); ++k) {
+      const LocRec &d = Q.recs[k];
+      const int64_t v[9] = {d.off, d.slice, d.u0, d.ncol, d.lower, d.head.loc0, d.head.lev, d.head.groups, d.head.nr};
+      std::copy(v, v + 9, recs + 9 * k);
     }
-  if (heads) std::copy(Q.heads.begin(), Q.heads.end(), heads);
-  for (int64_t i = 0; i < n && !P.fmap.empty() && !P.fmap[0].empty(); ++i) {
-    if (fmap) fmap[i] = P.fmap[0][size_t(i)];
-    if (bmap) bmap[i] = P.bmap[0][size_t(i)];
-  }
+  if (num && !P.lnum.empty()) std::copy(P.lnum[0].begin(), P.lnum[0].end(), num);
   return VSHE_OK;
 }
 

@@ -60,13 +60,13 @@ void vk_precond_copy(int ntiles, const void *sys, const void *st, const VkTiles 
 VK_DECL_P(float, f32)
 VK_DECL_P(double, f64)
 
-// the apply of block tasks whose solved values fit shared memory (trsv_local.cu), the slot of every
-// row, and columns in task numbers
-int vk_trsv_local(int mixed, int ntasks, int consumers, int ring, int stage_bytes, const void *sys, const void *st, const int32_t *act,
-                  const void *lsys, const void *tasks, const void *chunks, const void *copies, const void *heads, int which, const unsigned *bar,
-                  int32_t *err, cudaStream_t s);
-int vk_slots(int64_t n, const int64_t *dpos, int32_t *fslot, cudaStream_t s);
-int vk_map_columns(int64_t n, int64_t count, const int32_t *col, const int32_t *map, int32_t *out, cudaStream_t s);
+// the apply of block tasks whose solved values fit shared memory (trsv_local.cu), and the fill of one
+// system's records (sysdev: the host's SysDev): all = 1 everything, with the rows' numbers num, 0 the
+// factor's values
+int vk_trsv_local(int mixed, int ntasks, int nwarp, int ring, int slots, int slot_bytes, const void *sys, const void *st, const int32_t *act,
+                  const void *tasks, const void *runs, const void *warps, const void *recs, int which, const unsigned *bar, int32_t *err,
+                  cudaStream_t s);
+int vk_local_fill(int mixed, const void *sysdev, int nrec, const void *recs, const int32_t *num, int ring, int all, void *buf, cudaStream_t s);
 
 // the apply of whole systems with many short levels (trsv_stream.cu), and the fill of a system's stream
 // (sysdev: the host's SysDev): all = 1 its tables, 0 the factor's values; patch: (entry, shared-memory

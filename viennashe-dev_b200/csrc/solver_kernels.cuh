@@ -141,58 +141,53 @@ inline constexpr int64_t task_chunk_bytes(int64_t ns, int64_t nslot, int64_t r0,
   return 16 * ns + (4 + vbytes) * nslot + (r1 - r0) * (lower ? 8 : 4 + vbytes);
 }
 
-// Local sweep tasks (k_trsv_local): block tasks whose solved values fit shared memory.  A task
-// numbers its rows 0 .. m-1 in the order its forward sweep solves them, its backward slots likewise in
-// the order of the backward sweep; its factor columns are given in these numbers (LocSys), and the CTA
-// keeps value i at entry i of a shared-memory array of `ring` >= m entries.
-//
-// A chunk is a run of the task's slices, across levels, that fits one shared-memory stage:
-//   LocHead, int32 wptr[consumers + 1], SliceLoc[slices] (16-byte aligned; sorted by the
-//   consumer warp that sums them, wptr = each warp's range), factor columns, factor values, then
-//   per row operand, aligned runs of rows or slots one after the other: A = the input vector's rows
-//   (forward) or the forward result by slot (backward), FP64; B = the row's backward slot
-//   (forward) or the slot's row (backward); C = inverse diagonals (backward).
-// LocCopy lists the copies that fill it: bytes from (array `kind`) + src to stage offset dst.
-// Copies of the forward result come last (nlate) and wait for the forward sweep.
-struct LocTask {
-  int32_t sys, c0, nfwd, nchunk;  // chunks [c0, c0 + nchunk), the first nfwd forward
-  int32_t nlevF, nbar;            // forward levels; level barriers of the whole task
-  int32_t m, ring;
-};
+// Local sweep tasks (k_trsv_local): the same units as TaskDev, for block tasks whose solved values fit
+// shared memory.  A task numbers its rows 0 .. m-1 level by level of its forward sweep (LocRun: a level's
+// rows are consecutive); entry i of shared memory holds row i's input, then its forward and then its
+// backward result, each in the place of the one before.
+// The slices of a level are dealt to the task's warps by width, and a barrier ends every level.  Every warp
+// has its own sequence of records in chunks, which it copies itself into a ring of `slots`
+// shared-memory slots, slots - 1 chunks ahead.  A chunk is a LocChunk and records one after the other;
+// a record is up to kLocCols columns of a slice, four to a group:
+//   LocHead; per group P v[32][4] (factor values), then per group uint16 at[32][4] (numbers of the
+//   values they multiply, `ring` = a zero for padding); the last record of a backward slice also P
+//   dinv[32] (inverse diagonals), uint16 loc[32] (its rows' numbers).
+// k_local_fill writes them from the SELL slices (the values anew after every factorisation).
 struct LocChunk {
-  int32_t rec0, nrec, nlate;   // copies [rec0, rec0 + nrec), the last nlate after the forward sweep
-  int32_t bytes, late_bytes;   // of the first nrec - nlate copies, and of the others
-};
-struct LocCopy {
-  int64_t src;   // byte offset in the array of that kind
-  int32_t dst;   // byte offset in the stage
-  int32_t what;  // kind << 24 | bytes
-};
-enum LocKind { kLocHead = 0, kLocLCol, kLocLVal, kLocIn, kLocFSlot, kLocUCol, kLocUVal, kLocYSlot, kLocURow, kLocUDinv, kLocKinds };
-struct LocHead {
-  int32_t offA, offB, offC;  // stage offsets of the row operands
-  int32_t offD;              // stage offset of the slice descriptors
-  int32_t pass;              // level barriers to have passed before the next chunk is waited for
-  int32_t pad[3];
-};
-struct SliceLoc {
-  int32_t col, val;    // stage offsets of the slice's columns and values
-  int32_t op;          // index of its first row in the chunk's operand runs
-  int32_t wnr;         // width << 6 | rows
-  int32_t loc0, lev;   // number of its first row; level barriers to pass before its gathers
+  int32_t nrec, bytes_ahead;  // records; size of the chunk slots - 1 further on (0: none)
   int32_t pad[2];
 };
-// Per system of a batch: columns in task numbers (padding: kLocPad), backward slot of every row, and
-// the forward result by backward slot.
-constexpr int32_t kLocPad = 0x7fffffff;
-struct LocSys {
-  const int32_t *lcol, *ucol, *fslot;
-  double *yslot;
+struct LocHead {
+  int32_t loc0, lev;          // number of its first row (forward); level barriers to pass before its gathers
+  int32_t groups, nr;         // groups of columns; rows, 0: not the slice's last record, + kLocBack: backward
 };
-constexpr int kLocStages = 3;
-constexpr int kLocNarrow = 15, kLocWide = 31;  // most consumer warps with 128 and with 64 registers a thread
-constexpr int64_t kLocSmemMax = 229632;        // shared memory a CTA may ask for, less the kernel's static part
+constexpr int32_t kLocBack = 64;
+struct LocWarp {
+  int64_t off;                // byte offset of its first chunk
+  int32_t nchunk, bytes[3];   // chunks; sizes of the first
+};
+struct LocRun {
+  int32_t row, num;           // rows row .. of a forward level, their numbers num ..
+};
+struct LocTask {
+  int32_t sys, nlevF, nlev, m;      // forward levels; all levels; rows
+  int32_t warp0, run0, pad[2];      // its LocWarp from warp0 on, its LocRun [run0, run0 + nlevF)
+};
+// one record, or (slice < 0) a LocChunk, for k_local_fill
+struct LocRec {
+  int64_t off;
+  int32_t slice, u0, ncol;    // SELL slice, its columns [u0, u0 + ncol)
+  int32_t lower;              // 1: forward
+  LocHead head;
+};
+constexpr int32_t kLocPad = 0x7fffffff;  // a row without a task number
+constexpr int kLocWarps = 15, kLocSlots = 3, kLocCols = 8;
+constexpr int kLocStages = 3;            // shared-memory stages of k_trsv_stream
+constexpr int64_t kLocSmemMax = 229632;  // shared memory a CTA may ask for, less the kernels' static part
 inline constexpr int64_t local_smem_bytes(int64_t ring, int64_t stage_bytes) { return 8 * ring + 128 + kLocStages * stage_bytes; }
+inline constexpr int64_t local_rec_bytes(int64_t groups, bool dinv, int vbytes) {
+  return int64_t(sizeof(LocHead)) + 128 * groups * (2 + vbytes) + (dinv ? 32 * (2 + vbytes) : 0);
+}
 
 // Cluster sweep tasks (k_trsv_cluster): the same units as TaskDev, walked by one thread-block
 // cluster each, level by level, with the slices of level k of the forward (backward) sweep in

@@ -58,6 +58,11 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned by
                "l"(src), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
+// Asynchronous copy of 8 bytes into shared memory, and the wait for the thread's own copies.
+__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // Barrier of the consumer warps only (named barrier 1; the producer warp does not take part).
 __device__ __forceinline__ void consumers_sync(int nthreads) { asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory"); }
 

@@ -1,12 +1,18 @@
-// trsv_local.cu -- incomplete-LU apply of tasks whose solved values are gathered from shared memory
-// (k_trsv_local, the LocTask tables of solver_kernels.cuh).
+// trsv_local.cu -- incomplete-LU apply of block tasks whose solved values fit shared memory
+// (k_trsv_local; the records are described at LocHead in solver_kernels.cuh).
 //
-// k_trsv_task takes one chunk of copies per level and sends every gather of a solved value to L2 and
-// back.  On slabs of a few thousand rows that latency, not the bytes, sets the time.  Here a chunk
-// spans levels (one set of copies per 32 KB of operands, issued by the lanes of the producer warp in
-// parallel) and the solved values stay in shared memory.  Per apply, k_trsv_task before and
-// k_trsv_local now: 50x20x60 bar, L = 1 (38 tasks, 7 + 7 levels) 17.2 and 12.3 us, 100x25x80 bar,
-// L = 3 (52 tasks, 21 + 21 levels) 101 and 93 us.
+// On slabs of a few thousand rows k_trsv_task is bound by latency, not by bytes: a level is a handful of
+// slices per warp, every gather of a solved value goes to L2 and back, and all warps wait for each
+// chunk of copies together.  Here the values stay in shared memory, every warp streams its own slices
+// (bulk copies into its own slots, no hand-over between warps), and the warps meet only at the
+// level barriers.  Per apply, k_trsv_task and k_trsv_local: bar 50 x 20 x 60, first order (38 tasks of up
+// to 1040 rows) 17 and 9.0 us; bar 100 x 25 x 80, third order (52 of up to 15300) 101 and 76; bar 90 x
+// 29 x 64, third order (37 of up to 16008) 127 and 87; bar 71 x 27 x 67, third order, FP64 factors
+// (40 of up to 11826) 103 and 76.  What bounds the large ones is the chain of records of a warp, about 90
+// of 450 cycles for the gathers and sums and as many for the loads, beside a level's imbalance and shared memory
+// itself (a gather takes 3.8 passes over the banks); a task on a cluster of 2 to 4 CTAs, each with all
+// values, measured no better (86 to 100 us on the last but one: a level then waits for stores and
+// arrivals between SMs).
 #include <cuda_runtime.h>
 #include <cstdint>
 
@@ -18,270 +24,211 @@ namespace vshe {
 
 namespace {
 
-constexpr int kLocU = 4;  // entries of a row held in registers across the level barrier (rows of ILU(0) hold 2 to 5)
+extern __shared__ __align__(128) unsigned char l_smem[];
 
-// orders this thread's global writes before later bulk copies that read them (with the mbarrier
-// arrival that follows)
-__device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async;" ::: "memory"); }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, unsigned bytes) {
-  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-
-// What a warp reads of one slice from the stage before its level starts: lane = row.
+// a record in registers; columns past its groups are zeros times the zero of padding
 template <typename P>
-struct LocRow {
-  int4 d0, d1;  // SliceLoc
-  int dst;
-  double base;
+struct Record {
+  LocHead H;
+  uint2 at[2];
+  __align__(16) P v[8];
   P dinv;
-  int c[kLocU];
-  P v[kLocU];
-};
-
-// Barriers and source arrays of a task, by one thread.
-template <typename P>
-__device__ __forceinline__ void task_init(const SysDev<P> &S, const LocSys &Q, const unsigned char *heads, int which, int consumers,
-                                          const unsigned char **bases, uint64_t *full, uint64_t *empty, uint64_t *fwd) {
-  for (int i = 0; i < kLocStages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], consumers); }
-  mbar_init(fwd, consumers);
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  bases[kLocHead] = heads;
-  bases[kLocLCol] = (const unsigned char *)Q.lcol;
-  bases[kLocLVal] = (const unsigned char *)S.lval;
-  bases[kLocIn] = (const unsigned char *)(which == 0 ? S.p : S.s);
-  bases[kLocFSlot] = (const unsigned char *)Q.fslot;
-  bases[kLocUCol] = (const unsigned char *)Q.ucol;
-  bases[kLocUVal] = (const unsigned char *)S.uval;
-  bases[kLocYSlot] = (const unsigned char *)Q.yslot;
-  bases[kLocURow] = (const unsigned char *)S.urow;
-  bases[kLocUDinv] = (const unsigned char *)S.udinv;
-}
-
-// Everything of a slice that does not depend on the rows before it, from its stage (R.d0, R.d1 set).
-template <typename P>
-__device__ __forceinline__ void read_row(LocRow<P> &R, const unsigned char *stage, const LocHead &H, bool lower, int lane) {
-  const int width = R.d0.w >> 6;
-  const int32_t *c = (const int32_t *)(stage + R.d0.x) + lane;
-  const P *v = (const P *)(stage + R.d0.y) + lane;
+  int loc;
+  // loads the record at rec; returns the next
+  __device__ __forceinline__ const unsigned char *load(const unsigned char *rec, int lane, int ring) {
+    H = *(const LocHead *)rec;
+    rec += sizeof(LocHead);
+    const unsigned char *at_ = rec + 128 * sizeof(P) * H.groups;
 #pragma unroll
-  for (int u = 0; u < kLocU; ++u) {
-    R.c[u] = kLocPad; R.v[u] = P(0);
-    if (u < width) { R.c[u] = c[32 * u]; R.v[u] = v[32 * u]; }
-  }
-  R.base = 0.0; R.dinv = P(1); R.dst = 0;
-  if (lane < (R.d0.w & 63)) {
-    const int op = R.d0.z + lane;
-    R.base = ((const double *)(stage + H.offA))[op];
-    R.dst = ((const int32_t *)(stage + H.offB))[op];
-    if (!lower) R.dinv = ((const P *)(stage + H.offC))[op];
-  }
-}
-
-// The producer warp of a task: lane i issues copies i, i + 32, ... of a chunk.  Leaves once its
-// copies have landed.
-__device__ __forceinline__ void produce(const LocTask &T, const LocChunk *chunks, const LocCopy *copies, const unsigned char *const *bases,
-                                        unsigned char *stages, int stage_bytes, uint64_t *full, uint64_t *empty, uint64_t *fwd,
-                                        unsigned long long limit, int32_t *err) {
-  const int lane = threadIdx.x & 31;
-  int issued = 0;
-  bool fwd_done = false;
-  LocChunk next = T.nchunk > 0 ? chunks[T.c0] : LocChunk{};
-  for (int g = 0; g < T.nchunk; ++g) {
-    const LocChunk c = next;
-    if (g + 1 < T.nchunk) next = chunks[T.c0 + g + 1];
-    LocCopy r0{};
-    if (lane < c.nrec) r0 = copies[c.rec0 + lane];
-    const int e = *((volatile int32_t *)err);
-    const int stg = g % kLocStages, round = g / kLocStages;
-    bool ok = e == 0;
-    if (ok && round > 0 && lane == 0) ok = mbar_wait(&empty[stg], (round - 1) & 1, limit, err);
-    if (!__all_sync(0xffffffffu, ok)) break;
-    const bool late = c.nlate > 0 && !fwd_done;
-    const int now = late ? c.nrec - c.nlate : c.nrec;
-    if (lane == 0) {
-      if (late) mbar_expect_tx(&full[stg], (unsigned)c.bytes);
-      else mbar_arrive_expect_tx(&full[stg], (unsigned)(c.bytes + c.late_bytes));
-    }
-    __syncwarp();
-    unsigned char *base = stages + (size_t)stg * stage_bytes;
-    for (int i = lane; i < now; i += 32) {
-      const LocCopy r = i == lane ? r0 : copies[c.rec0 + i];
-      bulk_g2s(base + r.dst, bases[r.what >> 24] + r.src, (unsigned)(r.what & 0xffffff), &full[stg]);
-    }
-    issued = g + 1;
-    if (late) {
-      bool done = true;
-      if (lane == 0) done = mbar_wait(fwd, 0, limit, err);
-      done = __all_sync(0xffffffffu, done);
-      // (after a failed wait the phase still completes with the copies issued, for the drain below)
-      if (lane == 0) mbar_arrive_expect_tx(&full[stg], done ? (unsigned)c.late_bytes : 0u);
-      __syncwarp();
-      if (!done) break;
-      fence_async_proxy();
-      for (int i = now + lane; i < c.nrec; i += 32) {
-        const LocCopy r = copies[c.rec0 + i];
-        bulk_g2s(base + r.dst, bases[r.what >> 24] + r.src, (unsigned)(r.what & 0xffffff), &full[stg]);
+    for (int g = 0; g < 2; ++g) {
+      at[g] = make_uint2((unsigned)ring * 65537u, (unsigned)ring * 65537u);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[4 * g + u] = P(0);
+      if (g < H.groups) {
+        at[g] = *(const uint2 *)(at_ + 256 * g + 8 * lane);
+        const uint4 *q = (const uint4 *)(rec + g * 128 * sizeof(P) + 4 * sizeof(P) * lane);
+#pragma unroll
+        for (int u = 0; u < (int)sizeof(P) / 4; ++u) *(uint4 *)(v + 4 * g + u * 16 / (int)sizeof(P)) = q[u];
       }
-      fwd_done = true;
     }
+    rec = at_ + 256 * H.groups;
+    loc = H.loc0 + lane;
+    dinv = P(1);
+    if (H.nr >= kLocBack) {
+      dinv = ((const P *)rec)[lane];
+      loc = ((const uint16_t *)(rec + 32 * sizeof(P)))[lane];
+      rec += 32 * (sizeof(P) + 2);
+    }
+    return rec;
   }
-  __syncwarp();
-  // copies of the last kLocStages chunks can be in flight; leave once they have landed
-  if (lane == 0)
-    for (int g = issued > kLocStages ? issued - kLocStages : 0; g < issued; ++g) mbar_drain(&full[g % kLocStages], (g / kLocStages) & 1);
-}
+  __device__ __forceinline__ double sum(double s) const {
+    const double *val = (const double *)l_smem;
+    double x[8];
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      x[4 * g] = val[at[g].x & 0xffff];
+      x[4 * g + 1] = val[at[g].x >> 16];
+      x[4 * g + 2] = val[at[g].y & 0xffff];
+      x[4 * g + 3] = val[at[g].y >> 16];
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s = fma((double)v[u], x[u], s);
+    return s;
+  }
+};
 
 }  // namespace
 
-// The incomplete-LU apply of one task (a whole system or a run of preconditioner blocks) on one CTA:
-// out = U^{-1} L^{-1} in, level by level.  Slice by slice and row by row it is the arithmetic of
-// k_trsv_task (one row per lane, summed in index order with FP64 FMAs), so both give the same bits.
-//
-// One producer warp streams the task's chunks through kLocStages shared-memory stages.  The
-// consumer warps take the slices the plan assigned to them, a named barrier between two levels.  A
-// warp reads the columns, values and operands of its next slice from the stage before it sums
-// the current one (kMaxThreads <= 512; with 1024 threads the registers do not allow it, and
-// the other warps cover the latency), and the gathers older than the ring go out before the
-// level barrier, so between two barriers there are only the gathers from the ring, the FMAs and the store.
-// A warp waits for the next chunk only after it has passed the level barriers its predecessors in
-// the current chunk need (LocHead::pass), so chunk waits and level barriers cannot hold each other
-// up.  The forward result is written by backward slot (yslot): the backward sweep reads it in slot
-// order, so it is copied into the stages like every other operand, by bulk copies that the producer
-// issues once every consumer has fenced its writes (fwd).
-//
-// Every chunk wait is bounded (bar[2..3] polls).  After one has failed the error word is set, the
-// warp takes the remaining level barriers without touching the stages and leaves, the others
-// find the error word in their own waits, and the producer drains its copies in flight before it
-// leaves.
-template <typename P, int kMaxThreads>
-__global__ void __launch_bounds__(kMaxThreads, 1)
-    k_trsv_local(const SysDev<P> *sys, const BiState *st, const int32_t *active, const LocSys *lsys, const LocTask *tasks,
-                 const LocChunk *chunks, const LocCopy *copies, const unsigned char *heads, int which, int ring_max, int stage_bytes,
-                 const unsigned *bar, int32_t *err) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(8) uint64_t full[kLocStages], empty[kLocStages], fwd;
-  __shared__ const unsigned char *bases[kLocKinds];
+// out = U^{-1} L^{-1} in for one block task on one CTA.  The arithmetic of a row is that of k_trsv_task,
+// bit for bit.  Waits for copies are bounded (bar[2..3] polls); after one has failed the error word is
+// set, the warp takes the remaining barriers without touching its slots, waits for its copies in flight
+// and leaves; the others find the error word in their own waits.
+template <typename P>
+__global__ void __launch_bounds__(32 * kLocWarps, 1)
+    k_trsv_local(const SysDev<P> *sys, const BiState *st, const int32_t *active, const LocTask *tasks, const LocRun *runs, const LocWarp *warps,
+                 const unsigned char *recs, int which, int ring, int slots, int slot_bytes, const unsigned *bar, int32_t *err) {
+  __shared__ __align__(8) uint64_t full[kLocWarps * kLocSlots];
   const LocTask T = tasks[blockIdx.x];
   const int s = T.sys;
   if (!active[s] || st[s].done || (which == 1 && st[s].s_conv)) return;
   const SysDev<P> &S = sys[s];
-  const LocSys &Q = lsys[s];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, consumers = (int)(blockDim.x >> 5) - 1;
-  double *win = (double *)smem;
-  unsigned char *stages = smem + 8 * (size_t)ring_max + 128;
-  if (threadIdx.x == 0) {
-    task_init(S, Q, heads, which, consumers, bases, full, empty, &fwd);
-    win[ring_max] = 0.0;  // the value of padding entries
-  }
-  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, threads = (int)blockDim.x;
+  double *val = (double *)l_smem;
+  const LocWarp W = warps[T.warp0 + warp];
+  uint64_t *mine = full + warp * kLocSlots;
+  unsigned char *slot0 = l_smem + 8 * (size_t)ring + 128 + (size_t)(warp * slots) * slot_bytes;
   const unsigned long long limit = spin_limit_of(bar);
-
-  if (warp == consumers) {
-    produce(T, chunks, copies, bases, stages, stage_bytes, full, empty, &fwd, limit, err);
-    return;
+  const unsigned char *next = recs + W.off;  // lane 0: the next chunk to copy
+  int issued = 0;
+  auto issue = [&](int slot, int bytes) {
+    mbar_arrive_expect_tx(&mine[slot], (unsigned)bytes);
+    bulk_g2s(slot0 + slot * slot_bytes, next, (unsigned)bytes, &mine[slot]);
+    next += bytes;
+    ++issued;
+  };
+  if (lane == 0) {
+#pragma unroll
+    for (int i = 0; i < kLocSlots; ++i) mbar_init(&mine[i], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < kLocSlots - 1; ++i)
+      if (i < slots - 1 && i < W.nchunk) issue(i, W.bytes[i]);
   }
-
-  // consumers
-  constexpr bool kAhead = kMaxThreads <= 512;
-  const int zero = ring_max, m = T.m, threads = 32 * consumers;
-  double *out = which == 0 ? S.ph : S.sh, *yslot = Q.yslot;
-  int lev = 0;  // level barriers passed
-  auto pass_to = [&](int target) {
-    while (lev < target) {
-      consumers_sync(threads);
-      if (++lev == T.nlevF) {  // the forward result is complete: hand this thread's part to the bulk copies
-        fence_async_proxy();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&fwd);
+  // the input in the order of the numbers; a lane holds one level's run of rows
+  const double *in = which == 0 ? S.p : S.s;
+  double *out = which == 0 ? S.ph : S.sh;
+  auto each_run = [&](auto &&f) {
+    for (int k0 = 0; k0 < T.nlevF; k0 += 32) {
+      LocRun R{0, 0};
+      if (k0 + lane < T.nlevF) R = runs[T.run0 + k0 + lane];
+      int end = __shfl_down_sync(0xffffffffu, R.num, 1);
+      if (k0 + lane + 1 == T.nlevF) end = T.m;
+      else if (lane == 31 && k0 + 32 < T.nlevF) end = runs[T.run0 + k0 + 32].num;
+      for (int k = 0; k < 32 && k0 + k < T.nlevF; ++k) {
+        const int row = __shfl_sync(0xffffffffu, R.row, k), num = __shfl_sync(0xffffffffu, R.num, k);
+        f(row, num, __shfl_sync(0xffffffffu, end, k) - num);
       }
     }
   };
-  for (int g = 0; g < T.nchunk; ++g) {
-    const int stg = g % kLocStages;
-    const bool lower = g < T.nfwd;
-    if (!mbar_wait(&full[stg], (g / kLocStages) & 1, limit, err)) { pass_to(T.nbar); return; }
-    const unsigned char *stage = stages + (size_t)stg * stage_bytes;
-    const LocHead H = *(const LocHead *)stage;
-    const int32_t *wptr = (const int32_t *)(stage + sizeof(LocHead));
-    const int4 *sd = (const int4 *)(stage + H.offD);
-    auto read = [&](LocRow<P> &R) { read_row(R, stage, H, lower, lane); };
-    auto solve = [&](const LocRow<P> &R) {
-      const int width = R.d0.w >> 6, nr = R.d0.w & 63, loc = R.d1.x + lane;
-      int idx[kLocU];
-      double a[kLocU], x[kLocU];
-#pragma unroll
-      for (int u = 0; u < kLocU; ++u) {
-        const int q = R.c[u];
-        idx[u] = q >= m ? zero : q;
-        a[u] = (double)R.v[u];
-      }
-      pass_to(R.d1.y);
-      double sum = 0.0;
-#pragma unroll
-      for (int u = 0; u < kLocU; ++u)
-        if (u < width) x[u] = win[idx[u]];
-#pragma unroll
-      for (int u = 0; u < kLocU; ++u)
-        if (u < width) sum = fma(a[u], x[u], sum);
-      if (width > kLocU) {
-        const int32_t *c = (const int32_t *)(stage + R.d0.x) + lane;
-        const P *v = (const P *)(stage + R.d0.y) + lane;
-#pragma unroll 4
-        for (int k = kLocU; k < width; ++k) {
-          const int q = c[32 * k];
-          sum = fma((double)v[32 * k], win[q >= m ? zero : q], sum);
-        }
-      }
-      if (lane < nr) {
-        const double y = lower ? R.base - sum : (R.base - sum) * (double)R.dinv;
-        win[loc] = y;
-        (lower ? yslot : out)[R.dst] = y;
-      }
-    };
-    const int i1 = wptr[warp + 1];
-    int i = wptr[warp];
-    if constexpr (kAhead) {
-      LocRow<P> A, B;
-      int4 e0{}, e1{};  // the descriptor after the next
-      auto ahead = [&](LocRow<P> &R) {
-        if (i + 1 < i1) { R.d0 = e0; R.d1 = e1; read(R); }
-        if (i + 2 < i1) { e0 = sd[2 * i + 4]; e1 = sd[2 * i + 5]; }
-      };
-      if (i < i1) { A.d0 = sd[2 * i]; A.d1 = sd[2 * i + 1]; read(A); }
-      if (i + 1 < i1) { e0 = sd[2 * i + 2]; e1 = sd[2 * i + 3]; }
-      while (i < i1) {
-        ahead(B);
-        solve(A);
-        if (++i >= i1) break;
-        ahead(A);
-        solve(B);
-        ++i;
-      }
-    } else {
-      for (; i < i1; ++i) {
-        LocRow<P> R;
-        R.d0 = sd[2 * i]; R.d1 = sd[2 * i + 1];
-        read(R);
-        solve(R);
-      }
+  each_run([&](int row, int num, int n) {
+    for (int i = (int)threadIdx.x; i < n; i += threads) cp_async8(val + num + i, in + row + i);
+  });
+  if (threadIdx.x == 0) val[ring] = 0.0;
+  cp_async_wait_all();
+  __syncthreads();
+  // A record is loaded into registers before the one ahead of it is worked on, so that its loads pass
+  // behind that one's gathers and barriers.
+  Record<P> R0, R1;
+  int passed = 0, chunk = -1, slot = -1, phase = 0, left = 0, ahead = 0;
+  const unsigned char *rec = nullptr;
+  bool ok = true;
+  double sum = 0.0;
+  auto load = [&](Record<P> &R) {
+    if (left == 0) {
+      if (++chunk == W.nchunk) return false;
+      if (++slot == slots) { slot = 0; phase ^= 1; }
+      if (!(ok = mbar_wait(&mine[slot], phase, limit, err))) return false;
+      rec = slot0 + slot * slot_bytes;
+      const LocChunk C = *(const LocChunk *)rec;
+      rec += sizeof(LocChunk);
+      left = C.nrec;
+      ahead = C.bytes_ahead;
+    }
+    --left;
+    rec = R.load(rec, lane, ring);
+    return true;
+  };
+  auto work = [&](Record<P> &R) {
+    for (; passed < R.H.lev; ++passed) consumers_sync(threads);
+    const int nr = R.H.nr & (kLocBack - 1);
+    const double base = lane < nr ? val[R.loc] : 0.0;
+    sum = R.sum(sum);
+    if (nr) {
+      if (lane < nr) val[R.loc] = (base - sum) * (double)R.dinv;
+      sum = 0.0;
     }
     __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[stg]);
-    pass_to(H.pass);
+    // the slot before the one being read is free: its last record is done
+    if (ahead) {
+      if (lane == 0) issue(slot == 0 ? slots - 1 : slot - 1, ahead);
+      ahead = 0;
+    }
+  };
+  for (bool more = load(R0); more;) {
+    more = load(R1);
+    work(R0);
+    if (!more) break;
+    more = load(R0);
+    work(R1);
   }
+  if (!ok) {
+    for (; passed < T.nlev; ++passed) consumers_sync(threads);
+    if (lane == 0)
+      for (int q = chunk; q < issued; ++q) mbar_drain(&mine[q % slots], (q / slots) & 1);
+    __syncwarp();
+    return;
+  }
+  for (; passed < T.nlev; ++passed) consumers_sync(threads);
+  each_run([&](int row, int num, int n) {
+    for (int i = (int)threadIdx.x; i < n; i += threads) out[row + i] = val[num + i];
+  });
 }
 
-// slot of every row as int32
-__global__ void k_slots(int64_t n, const int64_t *dpos, int32_t *fslot) {
-  const int64_t step = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) fslot[i] = (int32_t)dpos[i];
-}
-// out[k] = map[col[k]], kLocPad for padding (column n)
-__global__ void k_map_columns(int64_t n, int64_t count, const int32_t *col, const int32_t *map, int32_t *out) {
-  const int64_t step = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < count; k += step) {
-    const int32_t c = col[k];
-    out[k] = c < n ? map[c] : kLocPad;
+// Records from the SELL slices, one warp per record.  all: everything, with the rows' numbers (num, by
+// solver row); else the factor's values only.
+template <typename P>
+__global__ void k_local_fill(SysDev<P> S, int nrec, const LocRec *recs, const int32_t *num, int ring, bool all, unsigned char *buf) {
+  const int lane = threadIdx.x & 31, nw = (int)(gridDim.x * blockDim.x >> 5);
+  for (int r = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); r < nrec; r += nw) {
+    const LocRec R = recs[r];
+    unsigned char *rec = buf + R.off;
+    if (all && lane == 0) *(LocHead *)rec = R.head;
+    if (R.slice < 0) continue;
+    const bool lower = R.lower != 0, back = R.head.nr >= kLocBack;
+    const int j = R.slice, W = 4 * R.head.groups, nr = R.head.nr & (kLocBack - 1);
+    const int64_t off = (lower ? S.loff[j] : S.uoff[j]) + 32 * R.u0 + lane;
+    rec += sizeof(LocHead);
+    P *v = (P *)rec + 4 * lane;
+    uint16_t *at = (uint16_t *)(rec + 32 * sizeof(P) * W) + 4 * lane;
+    unsigned char *tail = rec + 32 * (sizeof(P) + 2) * W;
+    const int32_t slot = lower ? 0 : S.uslot0[j] + lane;
+    for (int u = 0; u < W; ++u) {
+      const int e = 128 * (u >> 2) + (u & 3);
+      if (all) {
+        const int32_t c = u < R.ncol ? (lower ? S.lcol : S.ucol)[off + 32 * u] : (int32_t)S.n;
+        at[e] = (uint16_t)(c < S.n ? num[c] : ring);
+        v[e] = P(0);
+      } else if (u < R.ncol) {
+        v[e] = (lower ? S.lval : S.uval)[off + 32 * u];
+      }
+    }
+    if (!back) continue;
+    if (all) {
+      ((P *)tail)[lane] = P(1);
+      ((uint16_t *)(tail + 32 * sizeof(P)))[lane] = (uint16_t)(lane < nr ? num[S.urow[slot]] : ring);
+    } else if (lane < nr) {
+      ((P *)tail)[lane] = S.udinv[slot];
+    }
   }
 }
 
@@ -290,40 +237,39 @@ __global__ void k_map_columns(int64_t n, int64_t count, const int32_t *col, cons
 using namespace vshe;
 
 template <typename P>
-static int launch_local(int ntasks, int consumers, int ring, int stage_bytes, const void *sys, const void *st, const int32_t *act,
-                        const void *lsys, const void *tasks, const void *chunks, const void *copies, const void *heads, int which,
-                        const unsigned *bar, int32_t *err, cudaStream_t s) {
-  constexpr int narrow = 32 * (kLocNarrow + 1), wide = 32 * (kLocWide + 1);
-  const auto k = consumers > kLocNarrow ? k_trsv_local<P, wide> : k_trsv_local<P, narrow>;
-  const int smem = (int)local_smem_bytes(ring, stage_bytes);
-  cudaError_t e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLocSmemMax);
+static int launch_local(int ntasks, int nwarp, int ring, int slots, int slot_bytes, const void *sys, const void *st, const int32_t *act,
+                        const void *tasks, const void *runs, const void *warps, const void *recs, int which, const unsigned *bar,
+                        int32_t *err, cudaStream_t s) {
+  cudaError_t e = cudaFuncSetAttribute((const void *)k_trsv_local<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLocSmemMax);
   if (e != cudaSuccess) return (int)e;
   vk_count_launches(1);
-  k<<<ntasks, 32 * (consumers + 1), smem, s>>>((const SysDev<P> *)sys, (const BiState *)st, act, (const LocSys *)lsys, (const LocTask *)tasks,
-                                               (const LocChunk *)chunks, (const LocCopy *)copies, (const unsigned char *)heads, which, ring,
-                                               stage_bytes, bar, err);
+  k_trsv_local<P><<<ntasks, 32 * nwarp, 8 * ring + 128 + nwarp * slots * slot_bytes, s>>>(
+      (const SysDev<P> *)sys, (const BiState *)st, act, (const LocTask *)tasks, (const LocRun *)runs, (const LocWarp *)warps,
+      (const unsigned char *)recs, which, ring, slots, slot_bytes, bar, err);
+  return (int)cudaGetLastError();
+}
+
+template <typename P>
+static int launch_local_fill(const void *sysdev, int nrec, const void *recs, const int32_t *num, int ring, bool all, void *buf, cudaStream_t s) {
+  vk_count_launches(1);
+  const int blocks = nrec < 8 * 1184 ? (nrec + 7) / 8 : 1184;
+  k_local_fill<P><<<blocks, 256, 0, s>>>(*(const SysDev<P> *)sysdev, nrec, (const LocRec *)recs, num, ring, all, (unsigned char *)buf);
   return (int)cudaGetLastError();
 }
 
 extern "C" {
 
-int vk_trsv_local(int mixed, int ntasks, int consumers, int ring, int stage_bytes, const void *sys, const void *st, const int32_t *act,
-                  const void *lsys, const void *tasks, const void *chunks, const void *copies, const void *heads, int which, const unsigned *bar,
-                  int32_t *err, cudaStream_t s) {
-  return mixed ? launch_local<float>(ntasks, consumers, ring, stage_bytes, sys, st, act, lsys, tasks, chunks, copies, heads, which, bar, err, s)
-               : launch_local<double>(ntasks, consumers, ring, stage_bytes, sys, st, act, lsys, tasks, chunks, copies, heads, which, bar, err, s);
+int vk_trsv_local(int mixed, int ntasks, int nwarp, int ring, int slots, int slot_bytes, const void *sys, const void *st, const int32_t *act,
+                  const void *tasks, const void *runs, const void *warps, const void *recs, int which, const unsigned *bar, int32_t *err,
+                  cudaStream_t s) {
+  return mixed ? launch_local<float>(ntasks, nwarp, ring, slots, slot_bytes, sys, st, act, tasks, runs, warps, recs, which, bar, err, s)
+               : launch_local<double>(ntasks, nwarp, ring, slots, slot_bytes, sys, st, act, tasks, runs, warps, recs, which, bar, err, s);
 }
 
-int vk_slots(int64_t n, const int64_t *dpos, int32_t *fslot, cudaStream_t s) {
-  vk_count_launches(1);
-  k_slots<<<592, 256, 0, s>>>(n, dpos, fslot);
-  return (int)cudaGetLastError();
-}
-
-int vk_map_columns(int64_t n, int64_t count, const int32_t *col, const int32_t *map, int32_t *out, cudaStream_t s) {
-  vk_count_launches(1);
-  k_map_columns<<<592, 256, 0, s>>>(n, count, col, map, out);
-  return (int)cudaGetLastError();
+int vk_local_fill(int mixed, const void *sysdev, int nrec, const void *recs, const int32_t *num, int ring, int all, void *buf, cudaStream_t s) {
+  if (nrec <= 0) return 0;
+  return mixed ? launch_local_fill<float>(sysdev, nrec, recs, num, ring, all != 0, buf, s)
+               : launch_local_fill<double>(sysdev, nrec, recs, num, ring, all != 0, buf, s);
 }
 
 }  // extern "C"

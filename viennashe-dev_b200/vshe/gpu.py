@@ -137,8 +137,7 @@ def sweep_plan(rp, ci, values=None, num_sms=148, **kw):
 
 def local_plan(rp, ci, values=None, num_sms=148, **kw):
     """vshe_layout_local_plan: the local tasks of one system's sweep plan (host only) -> dict of the
-    launch shape and the tables "tasks" (t, 8), "chunks" (c, 5), "copies" (k, 4), "heads" (bytes),
-    "fmap", "bmap" (n)."""
+    launch shape and the tables "tasks" (t, 6), "runs" (k, 2), "warps" (w, 5), "recs" (r, 9), "num" (n)."""
     L = lib()
     rp = np.ascontiguousarray(rp, np.int64)
     ci = np.ascontiguousarray(ci, np.int32)
@@ -146,19 +145,18 @@ def local_plan(rp, ci, values=None, num_sms=148, **kw):
     o, keep = make_opts(**kw)
     vals = None if values is None else np.ascontiguousarray(values, np.float64)
     L.vshe_layout_local_plan.argtypes = [C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(SolveOptsC),
-                                         C.c_int32] + [C.c_void_p] * 7
-    cnt = np.zeros(9, np.int64)
+                                         C.c_int32] + [C.c_void_p] * 6
+    cnt = np.zeros(10, np.int64)
     args = (n, int(rp[-1]), rp.ctypes.data, ci.ctypes.data, None if vals is None else vals.ctypes.data, C.byref(o), int(num_sms))
-    rc = L.vshe_layout_local_plan(*args, cnt.ctypes.data, *[None] * 6)
+    rc = L.vshe_layout_local_plan(*args, cnt.ctypes.data, *[None] * 5)
     if rc:
         raise VsheError(rc, "vshe_layout_local_plan")
-    t = {"tasks": np.zeros((int(cnt[0]), 8), np.int32), "chunks": np.zeros((int(cnt[1]), 5), np.int32),
-         "copies": np.zeros((int(cnt[2]), 4), np.int64), "heads": np.zeros(int(cnt[3]), np.uint8),
-         "fmap": np.zeros(n, np.int32), "bmap": np.zeros(n, np.int32)}
-    rc = L.vshe_layout_local_plan(*args, cnt.ctypes.data, *[t[k].ctypes.data for k in ("tasks", "chunks", "copies", "heads", "fmap", "bmap")])
+    t = {"tasks": np.zeros((int(cnt[0]), 6), np.int32), "runs": np.zeros((int(cnt[9]), 2), np.int32),
+         "warps": np.zeros((int(cnt[1]), 5), np.int64), "recs": np.zeros((int(cnt[2]), 9), np.int64), "num": np.zeros(n, np.int32)}
+    rc = L.vshe_layout_local_plan(*args, cnt.ctypes.data, *[t[k].ctypes.data for k in ("tasks", "runs", "warps", "recs", "num")])
     if rc:
         raise VsheError(rc, "vshe_layout_local_plan")
-    t.update(zip(("consumers", "ring", "stage", "rest"), (int(v) for v in cnt[4:])))
+    t.update(zip(("bytes", "nwarp", "ring", "slots", "slot_bytes", "rest"), (int(v) for v in cnt[3:])))
     return t
 
 
