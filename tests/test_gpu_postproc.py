@@ -39,3 +39,22 @@ def test_densities_and_currents_match_oracle(gpu_ctx, name):
     assert np.max(np.abs(dens - dens_r)) <= 1e-13 * np.max(np.abs(dens_r))
     assert len(cur) == len(cur_r)
     assert np.max(np.abs(cur - cur_r)) <= 1e-11 * cases.current_scale(dens_r, cur_r)
+
+
+def test_large_result_arrives_whole():
+    """x_full of 74 MB, downloaded in parts by several threads: the residual of the full system, from
+    the exported matrix, is the one the device reports (both FP64 sums over the rows; a part that
+    is missing or misplaced changes it by orders of magnitude)."""
+    dev, cfg = D.config2(100, 25, 240, 3)
+    ctx = gpu.Context(0)
+    try:
+        G = gpu.SheProblem(ctx, dev, cfg, precond="block_ilu0", ordering="multicolor", fill_level=0, tol=1e-4)
+        full_residual = G.run()[1]
+        rp, ci, val, rhs = G.export("full")
+        for _ in range(2):  # allocates the staging buffers, then uses them again
+            x = G.results()[0]
+            assert x.nbytes > 64 << 20
+            r = np.linalg.norm(np.add.reduceat(val * x[ci], rp[:-1]) - rhs) / np.linalg.norm(rhs)
+            assert r == pytest.approx(full_residual, rel=1e-6)
+    finally:
+        ctx.close()
