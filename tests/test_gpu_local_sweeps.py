@@ -65,7 +65,7 @@ def test_stream_equals_task(precision, n, offsets):
     ([3000] * 170, [-60, -1, 1, 60]),                                   # more blocks than tasks
     ([16384, 16385, 200, 16000], [-128, -1, 1, 128]),                   # long levels: k_trsv_task
     # below and above what fits shared memory
-    ([19800, 20000, 23500, 23700, 16000], [-700, -251, -250, -126, -125, -3, -2, -1, 1, 2, 3, 125, 126, 250, 251, 700]),
+    *[(sizes, [-700, -251, -250, -126, -125, -3, -2, -1, 1, 2, 3, 125, 126, 250, 251, 700]) for sizes in ([12200, 9000], [12400, 9000], [18700, 16000], [18900, 16000])],
 ])
 def test_local_equals_task(precision, sizes, offsets):
     blocks = np.concatenate([[0], np.cumsum(sizes)])

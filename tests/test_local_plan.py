@@ -248,7 +248,7 @@ def test_local_plan_runs_like_the_level_sweep(name, num_sms):
     P = gpu.local_plan(rp, ci, vals, num_sms=num_sms, **kw)
     n, ring, nw, slots, sb = lay["n"], P["ring"], P["nwarp"], P["slots"], P["slot_bytes"]
     vb = np.dtype(vt).itemsize
-    assert 1 <= nw <= 15 and 2 <= slots <= 3 and ring % 16 == 0 and ring < 1 << 16 and sb % 16 == 0
+    assert 1 <= nw <= 15 and slots == 3 and ring % 16 == 0 and ring < 1 << 16 and sb % 16 == 0
     assert 8 * ring + 128 + nw * slots * sb + 1024 <= SMEM
     assert len(P["tasks"]) and P["rest"] == 0 and len(P["warps"]) == nw * len(P["tasks"])
     # the chunks and records as k_local_fill writes them, by offset; they follow each other without a gap

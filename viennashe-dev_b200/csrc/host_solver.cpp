@@ -1269,14 +1269,16 @@ static void add_local_task(const std::vector<System *> &sys, int vb, SweepPlan &
 }
 
 // Splits the tasks by kernel.  Whole systems with a stream take k_trsv_stream.  A block task is local
-// (k_trsv_local) if its values fit shared memory beside the slots of 12 warps, about 23,000 rows (FP64
-// factors 20,000; larger ones, energy slabs of large 2D meshes, keep k_trsv_task), and an average level has at most
-// 48 slices: beyond, k_trsv_task has enough gathers in flight, and more bandwidth (tasks of 16000 rows and
-// 125 slices a level 29 us per apply against 32, 8000 rows and 62 slices 21 against 18; of 21800 rows and 8
-// neighbours 186 against 149 with 15 warps, FP64 210 against 219 with 9).  One shape serves the batch: values for the largest local task; half
-// as many warps again as an average level has slices, since the slices' widths differ (bar 50 x 20 x
-// 60, 5 slices: 9.8 us per apply with 5 warps, 9.0 with 8, 9.1 with 10; bar 90 x 29 x 64, 14 slices:
-// 97 with 12, 87 with 15); and three slots of chunks per warp, two if they do not fit.
+// (k_trsv_local) if its values fit shared memory beside three slots of 15 warps, 18,800 rows (FP64
+// factors 12,300; with two slots a warp waits for its copies: bar 120 x 30 x 70, 22,000 rows 167 us per
+// apply against 117, bar 110 x 28 x 70, FP64, 18,800 rows 174 against 125), and an average level has at
+// most 48 slices: beyond, k_trsv_task has enough gathers in flight, and more bandwidth (tasks of 16000
+// rows and 125 slices a level 29 us against 32, 8000 rows and 62 slices 21 against 18).  A batch's block
+// tasks are local all or none: two kernels run one after the other, where one runs its tasks side by
+// side (a bar with slabs on both sides of the line: 243 ms a pass against 162).
+// One shape serves the batch: values for the largest local task; half as many warps again as an
+// average level has slices, since the slices' widths differ (bar 50 x 20 x 60, 5 slices: 9.8 us per
+// apply with 5 warps, 9.0 with 8, 9.1 with 10; bar 90 x 29 x 64, 14 slices: 97 with 12, 87 with 15).
 static void plan_local_tasks(const std::vector<System *> &sys, bool mixed, SweepPlan &P) {
   const int vb = mixed ? 4 : 8;
   const size_t nt = P.tasks.size();
@@ -1306,22 +1308,24 @@ static void plan_local_tasks(const std::vector<System *> &sys, bool mixed, Sweep
       }
     }
   }
-  constexpr int64_t kMinWarps = 12;
   constexpr double kMostSlices = 48;
   const int64_t slot = int64_t(sizeof(LocChunk)) + local_rec_bytes(kLocCols / 4, true, vb);
   std::vector<char> kind(nt, 0);  // 0 neither, 1 local, 2 stream
   double slices = 0, levels = 0;
   int64_t most = 1;
+  bool fit = true;
   for (size_t t = 0; t < nt; ++t) {
     const Info &I = info[t];
     const size_t k = size_t(P.ctasks[t].sys);
     if (P.on_task[k] == 1) { kind[t] = sys[k]->stream.ok ? 2 : 0; continue; }
-    if (8 * ((I.m + 15) & ~int64_t(15)) + 128 + kMinWarps * 2 * slot > kLocSmemMax || I.slices > kMostSlices * I.levels) continue;
+    fit = fit && 8 * ((I.m + 15) & ~int64_t(15)) + 128 + kLocWarps * kLocSlots * slot <= kLocSmemMax && I.slices <= kMostSlices * I.levels;
     kind[t] = 1;
     most = std::max(most, I.m);
     slices += I.slices;
     levels += I.levels;
   }
+  if (!fit)
+    for (char &k : kind) k = k == 1 ? 0 : k;
   std::vector<TaskDev> tk;
   std::vector<ClusterTask> ct;
   std::vector<size_t> order;
@@ -1339,8 +1343,8 @@ static void plan_local_tasks(const std::vector<System *> &sys, bool mixed, Sweep
   L.ring = int((most + 15) & ~int64_t(15));
   const int64_t left = kLocSmemMax - 8 * int64_t(L.ring) - 128;
   const int64_t want = std::max<int64_t>(1, int64_t(std::ceil(1.5 * slices / std::max(levels, 1.0))));
-  L.nwarp = int(std::min(std::min<int64_t>(want, kLocWarps), left / (2 * slot)));
-  L.slots = left >= 3 * slot * L.nwarp ? 3 : 2;
+  L.nwarp = int(std::min<int64_t>(want, kLocWarps));
+  L.slots = kLocSlots;
   L.slot_bytes = int(std::min<int64_t>(left / (L.slots * L.nwarp), 8192) & ~int64_t(15));
   // the tasks of a member one after the other, so that its records are one run
   for (size_t k = 0; k < sys.size(); ++k) {
