@@ -11,7 +11,7 @@
 // (40 of up to 11826) 103 and 76.  What bounds the large ones is the chain of records of a warp, about 90
 // of 450 cycles for the gathers and sums and as many for the loads, beside a level's imbalance and shared memory
 // itself (a gather takes 3.8 passes over the banks); a task on a cluster of 2 to 4 CTAs, each with all
-// values, measured no better (86 to 100 us on the last but one: a level then waits for stores and
+// values, measured no better (87 to 100 us on the third of these: a level then waits for stores and
 // arrivals between SMs).
 #include <cuda_runtime.h>
 #include <cstdint>
