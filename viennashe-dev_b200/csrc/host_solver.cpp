@@ -1369,8 +1369,9 @@ static void plan_local_tasks(const std::vector<System *> &sys, bool mixed, Sweep
 // The stream of a system swept as one task: the slices of each level dealt to nwarp warps in steps, the
 // steps cut into chunks.  A warp's slices of a sweep are stored at one width, their widest's (the
 // kernel's variant for it; a level's slices come widest first, so the later warps get narrow ones);
-// beyond kStreamW a slice keeps its own.  No stream where a slice does not fit a stage or three
-// consecutive chunks or levels do not fit the ring.
+// beyond kStreamW a slice keeps its own.  No stream where a slice does not fit a stage, a level
+// does not fit the ring, or a value that has left the ring may still be in work when its reader's chunk is
+// fetched.
 void plan_stream(const System &S, const Layout &L, StreamPlan &P) {
   P = StreamPlan{};
   const int eb = S.mixed ? int(sizeof(StreamEnt<float>)) : int(sizeof(StreamEnt<double>));
@@ -1420,7 +1421,6 @@ void plan_stream(const System &S, const Layout &L, StreamPlan &P) {
     const bool lower = pass == 0;
     const std::vector<int64_t> &off = lower ? S.loff_h : S.uoff_h, &rs = lower ? S.lrow0_h : S.uslot0_h, &lv = lower ? S.lvsL : S.lvsU;
     const std::vector<int32_t> &col = lower ? L.lcol : L.ucol;
-    const size_t first = P.chunks.size();
     std::vector<int64_t> start;  // number of each chunk's first row
     auto stored = [&](int64_t j, int64_t warp) -> int64_t {
       const int w = P.width[pass][warp];
@@ -1463,7 +1463,11 @@ void plan_stream(const System &S, const Layout &L, StreamPlan &P) {
         r += 32 * int64_t(sizeof(StreamRow));
       }
       const int64_t stage0 = 8 * int64_t(P.ring) + 128 + int64_t(P.chunks.size() % kLocStages) * P.stage;
+      // the values older than the ring are copied when the chunk is fetched: every warp has then left the
+      // chunks up to the third before it, so a value must lie in one of those
+      const int64_t left = start.size() >= 2 ? start[start.size() - 2] : 0;
       for (size_t k = 0; k < old.size(); ++k) {
+        if (old[k].number >= left) fits = false;
         P.olds.push_back(old[k].number);
         P.patch.push_back(at[size_t(old[k].item)] + old[k].entry);
         P.patch.push_back(stage0 + at_old + 8 * int64_t(k));
@@ -1510,10 +1514,6 @@ void plan_stream(const System &S, const Layout &L, StreamPlan &P) {
     }
     flush();
     if (lower) P.nfwd = int(P.chunks.size());
-    // a value older than the ring lies in chunks before the two preceding its reader's
-    start.push_back(S.n);
-    for (size_t g = 0; first + g < P.chunks.size(); ++g)
-      if (P.keep[pass] && start[g + 1] - start[g < 2 ? 0 : g - 2] > P.ring) return;
   }
   if (!fits) return;
   for (size_t k = 0; k + 1 < S.lvsL.size(); ++k)  // rows of a level and the ring

@@ -203,8 +203,8 @@ struct ClusterTask {
 // Row i of a sweep (forward: the solver row, backward: the slot) keeps its value at i mod `ring` of a
 // shared-memory ring.  An entry whose column is older than the ring when its level ends (number below
 // level end - ring) is read from its chunk's stage, where the producer gathers such values from global
-// memory: the rows of three consecutive chunks fit the ring, so they are solved and written by all
-// warps when the chunk is fetched.
+// memory when it fetches the chunk.  Every warp is then through the chunks up to the third before it, and
+// plan_stream takes no stream where such a value lies in a later one (a level may span several chunks).
 //
 // Device arrays, filled by k_stream_fill (the values anew after every factorisation) from the SELL slices:
 //   entries: for slice record r, w entries of 32 lanes: StreamEnt (shared-memory byte offset of the
