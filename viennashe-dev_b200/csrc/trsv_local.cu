@@ -158,6 +158,13 @@ __global__ void __launch_bounds__(32 * kLocWarps, 1)
     rec = R.load(rec, lane, ring);
     return true;
   };
+  // the copy that opening a chunk asks for: the slot before it is free, its last record is done
+  auto copy_ahead = [&]() {
+    if (ahead) {
+      if (lane == 0) issue(slot == 0 ? slots - 1 : slot - 1, ahead);
+      ahead = 0;
+    }
+  };
   auto work = [&](Record<P> &R) {
     for (; passed < R.H.lev; ++passed) consumers_sync(threads);
     const int nr = R.H.nr & (kLocBack - 1);
@@ -168,13 +175,12 @@ __global__ void __launch_bounds__(32 * kLocWarps, 1)
       sum = 0.0;
     }
     __syncwarp();
-    // the slot before the one being read is free: its last record is done
-    if (ahead) {
-      if (lane == 0) issue(slot == 0 ? slots - 1 : slot - 1, ahead);
-      ahead = 0;
-    }
+    copy_ahead();
   };
-  for (bool more = load(R0); more;) {
+  bool more = load(R0);
+  // (chunk 0's goes into the slot not used yet: loading the second record may open chunk 1)
+  copy_ahead();
+  while (more) {
     more = load(R1);
     work(R0);
     if (!more) break;
