@@ -44,6 +44,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, unsign
   }
   return true;
 }
+// The same for a whole warp, whose lanes all learn the same outcome: what follows a failed wait (barriers
+// of the CTA, warp-wide instructions) must not find the warp split.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, unsigned parity, unsigned long long limit, int32_t *err) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit, err));
+}
 // Waits for a phase regardless of the error word, at most kDrainPolls polls: copies in flight
 // complete within microseconds, and shared memory must not be released under them.
 constexpr unsigned long long kDrainPolls = 1ull << 24;

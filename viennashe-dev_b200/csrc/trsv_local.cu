@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(32 * kLocWarps, 1)
     if (left == 0) {
       if (++chunk == W.nchunk) return false;
       if (++slot == slots) { slot = 0; phase ^= 1; }
-      if (!(ok = mbar_wait(&mine[slot], phase, limit, err))) return false;
+      if (!(ok = mbar_wait_warp(&mine[slot], phase, limit, err))) return false;
       rec = slot0 + slot * slot_bytes;
       const LocChunk C = *(const LocChunk *)rec;
       rec += sizeof(LocChunk);

@@ -122,7 +122,7 @@ __device__ __noinline__ bool walk(const Walk &wk) {
     // operand offsets count from the stage's start: the row at stage offset o is number
     // op0 + (o - first operand's offset) / 8
     double *keep = kKeep ? ytmp + chunks[g].op0 - ((chunks[g].head_bytes + chunks[g].ent_bytes + chunks[g].row_bytes) >> 3) - chunks[g].nold : nullptr;
-    if (!mbar_wait(&full[stg], (g / kLocStages) & 1, limit, err)) {
+    if (!mbar_wait_warp(&full[stg], (g / kLocStages) & 1, limit, err)) {
       // the error word is set or this wait ran out: every warp takes the level barriers that are left
       for (int q = g; q < g1; ++q)
         for (int b = 0; b < chunks[q].nstep; ++b) consumers_sync(threads);
