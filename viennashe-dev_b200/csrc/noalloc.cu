@@ -80,24 +80,23 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_al
 // kernel is bound by HBM (12 bytes an entry, 32 a row): a tile's entries are one contiguous run, so
 // the block's threads copy it to shared memory coalesced and asynchronously, the next tile's run
 // while they sum the current one, and each thread sums one row from there, in index order with
-// FMAs; the x gathers of neighbouring rows fall into the same lines.  A tile that averages more
-// than kWideRow entries a row is summed by warps instead, lanes striding a row, so that a dense
-// row does not wait on one thread.  Before, a warp walked a row at a time and 256 rows in series
+// FMAs; the x gathers of neighbouring rows fall into the same lines.  A row of more than kLongRow
+// entries is summed by its warp instead, lanes striding it, so that it does not wait on one thread,
+// whatever the rows around it.  Before, a warp walked a row at a time and 256 rows in series
 // (10 of its 32 lanes busy, three dependent loads a row).  Rows of 9 entries, before and now:
 // 1000 rows 94 and 6.3 us, 100 003 rows 199 and 10.3 us, 1 000 003 rows 310 and 42.6 us
 // (3.5 TB/s), 8 M rows 1271 and 290 us (4.1 TB/s).  Tiles of 256 rows, three blocks an SM: 49 and
 // 329 us on the last two; one buffer instead of two: 48 and 329 us.
 // The last block to finish adds the block partials in block order; the order of every sum is fixed
-// by n and the SM count.
-constexpr int64_t kWideRow = 32;
+// by the matrix and the SM count.
+constexpr int kLongRow = 48;
 __global__ void __launch_bounds__(kThreads, kBlocksPerSm) k_residual_noalloc(int64_t n, const int64_t *__restrict__ rp, const int32_t *__restrict__ ci,
                                                                              const double *__restrict__ av, const double *__restrict__ x,
                                                                              const double *__restrict__ b, double *__restrict__ r,
                                                                              double *__restrict__ norms2, NoAllocScratch *sc) {
   __shared__ double sval[2][kChunk];
   __shared__ int32_t scol[2][kChunk];
-  __shared__ double ssum[kRows];
-  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int t = threadIdx.x, lane = t & 31;
   const int64_t step = (int64_t)gridDim.x * kRows;
   // copies the first chunk of entries [e0, e1) into a buffer
   auto fetch = [&](int buf, int64_t e0, int64_t e1) {
@@ -119,9 +118,8 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) k_residual_noalloc(int
     const bool mine = t < rows;
     const int64_t a = mine ? rp[r0 + t] : 0, z = mine ? rp[r0 + t + 1] : 0;
     const double bi = mine ? b[r0 + t] : 0.0;
-    const bool wide = e1 - e0 > kWideRow * rows;
+    const bool longrow = z - a > kLongRow;
     double s = 0.0;
-    if (wide) ssum[t] = 0.0;
     cp_async_wait();
     __syncthreads();  // the tile's first chunk has landed, and the other buffer's readers are through
     int64_t g0 = 0, g1 = 0;
@@ -135,23 +133,21 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) k_residual_noalloc(int
         cp_async_wait();
         __syncthreads();
       }
-      if (!wide) {
-        const int64_t k1 = (z < base + m ? z : base + m) - base;
+      const int k0 = (int)((a < base ? base : a < base + m ? a : base + m) - base);
+      const int k1 = (int)((z < base ? base : z < base + m ? z : base + m) - base);
+      if (!longrow) {
 #pragma unroll 4
-        for (int64_t k = (a > base ? a : base) - base; k < k1; ++k) s = fma(sval[buf][k], x[scol[buf][k]], s);
-      } else {
-        for (int i = w; i < rows; i += kWarps) {
-          const int64_t ra = rp[r0 + i], rz = rp[r0 + i + 1];
-          const int64_t k1 = (rz < base + m ? rz : base + m) - base;
-          double p = 0.0;
+        for (int k = k0; k < k1; ++k) s = fma(sval[buf][k], x[scol[buf][k]], s);
+      }
+      for (unsigned of = __ballot_sync(0xffffffffu, longrow && k0 < k1); of; of &= of - 1) {
+        const int l = __ffs(of) - 1, q0 = __shfl_sync(0xffffffffu, k0, l), q1 = __shfl_sync(0xffffffffu, k1, l);
+        double p = 0.0;
 #pragma unroll 4
-          for (int64_t k = (ra > base ? ra : base) - base + lane; k < k1; k += 32) p = fma(sval[buf][k], x[scol[buf][k]], p);
-          p = warp_sum(p);
-          if (lane == 0) ssum[i] += p;
-        }
+        for (int k = q0 + lane; k < q1; k += 32) p = fma(sval[buf][k], x[scol[buf][k]], p);
+        p = warp_sum(p);
+        if (lane == l) s += p;
       }
     }
-    if (wide) { __syncthreads(); s = mine ? ssum[t] : 0.0; }
     if (mine) {
       const double ri = bi - s;
       r[r0 + t] = ri;
