@@ -1372,16 +1372,35 @@ static void plan_local_tasks(const std::vector<System *> &sys, bool mixed, Sweep
 // beyond kStreamW a slice keeps its own.  No stream where a slice does not fit a stage, a level
 // does not fit the ring, or a value that has left the ring may still be in work when its reader's chunk is
 // fetched.
+//
+// Nor where k_trsv_task is the sooner.  A chunk takes about 1.4 us from its stage's release to its last
+// step, whatever it holds up to 11 steps of 0.12 us, and an older value 7.5 ns of the producer's time;
+// k_trsv_task's level takes 0.85 us, and more with its slices and their width.  us per apply of stream and
+// task, FP32 factor: diode of 200 boxes, third order (7 slices a level) 576 and 1418; levels of 1, 8, 24, 48,
+// 64 and 96 narrow slices 1 : 6.0, 3.7, 1.4, 1.11, 0.94 and 0.85; natural-order bars 50 x 20 x 60, first
+// order (1680 older values) 115 and 161, 100 x 25 x 80, first order (33 thousand) 608 and 381, third order
+// (1.7 million) 27649 and 2255.  FP64 factor: the diode 1188 and 1375; levels of 16, 24, 32 and 48 slices
+// 1 : 1.21, 1.05, 1.0 and 0.89; the first bar 212 and 168.  A stream of a few chunks is as short as a launch.
+constexpr double kStreamChunkUs = 1.4, kStreamStepUs = 0.12, kStreamOldUs = 0.0075;
+constexpr double kTaskLevelUs = 0.85, kTaskSliceUs = 0.02, kTaskWidthUs = 0.012;
+constexpr size_t kStreamFewChunks = 8;
+
 void plan_stream(const System &S, const Layout &L, StreamPlan &P) {
   P = StreamPlan{};
   const int eb = S.mixed ? int(sizeof(StreamEnt<float>)) : int(sizeof(StreamEnt<double>));
-  double slices = 0, levels = 0;
+  double slices = 0, levels = 0, widths = 0;  // widths: of every level's widest slice
   for (int pass = 0; pass < 2; ++pass) {
-    const std::vector<int64_t> &lv = pass == 0 ? S.lvsL : S.lvsU;
+    const std::vector<int64_t> &off = pass == 0 ? S.loff_h : S.uoff_h, &lv = pass == 0 ? S.lvsL : S.lvsU;
     slices += double(lv.empty() ? 0 : lv.back() - lv.front());
     levels += double(lv.empty() ? 0 : lv.size() - 1);
+    for (size_t k = 0; k + 1 < lv.size(); ++k) {
+      int64_t w = 0;
+      for (int64_t j = lv[k]; j < lv[k + 1]; ++j) w = std::max(w, (off[size_t(j) + 1] - off[size_t(j)]) >> 5);
+      widths += double(w);
+    }
   }
   if (levels == 0 || S.n >= (int64_t(1) << 30)) return;
+  const double task_us = kTaskLevelUs * levels + kTaskSliceUs * slices + kTaskWidthUs * widths;
   // one slice per warp on most levels: fewer warps make the barrier cheaper, more steps per level cost more
   P.nwarp = 1;
   while (P.nwarp < kStreamWarps && double(P.nwarp) < 0.95 * slices / levels) P.nwarp = std::min(2 * P.nwarp, kStreamWarps);
@@ -1416,6 +1435,9 @@ void plan_stream(const System &S, const Layout &L, StreamPlan &P) {
     while (P.ring > 32 && local_smem_bytes(P.ring, P.stage) > kLocSmemMax) P.ring /= 2;
   }
   if (one > P.stage) return;
+  // (the fewest chunks the slices can take, before their older values are looked for)
+  const double least = (eb * double(S.padL + S.padU) + (32.0 * sizeof(StreamRow) + 256.0) * slices) / P.stage;
+  if (least > double(kStreamFewChunks) && kStreamChunkUs * least > task_us) return;
   bool fits = true;
   for (int pass = 0; pass < 2; ++pass) {
     const bool lower = pass == 0;
@@ -1516,6 +1538,9 @@ void plan_stream(const System &S, const Layout &L, StreamPlan &P) {
     if (lower) P.nfwd = int(P.chunks.size());
   }
   if (!fits) return;
+  double stream_us = kStreamOldUs * double(P.patch.size() / 2);
+  for (const StreamChunk &c : P.chunks) stream_us += std::max(kStreamChunkUs, kStreamStepUs * c.nstep);
+  if (P.chunks.size() > kStreamFewChunks && stream_us > task_us) return;
   for (size_t k = 0; k + 1 < S.lvsL.size(); ++k)  // rows of a level and the ring
     if (S.lrow0_h[size_t(S.lvsL[k + 1])] - S.lrow0_h[size_t(S.lvsL[k])] > P.ring) return;
   for (size_t k = 0; k + 1 < S.lvsU.size(); ++k)
