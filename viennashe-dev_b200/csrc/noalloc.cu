@@ -91,7 +91,8 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_al
 // by the matrix and the SM count.
 // Four partial sums are no less accurate than a warp that strides the row and adds its lanes up in a tree
 // up to 28 entries (root mean square error of 28: 5.6 against 5.7 units of 2^-53; one running sum 8.6),
-// eight up to 48 (7.6 against 7.7; four 8.6).
+// eight up to 48 (7.6 against 7.7; four 8.6).  Each row chooses for itself: where a warp chose for its rows,
+// rows of 22 to 33 entries took 119 us instead of 107, of 33 to 47 154 instead of 121 (500 000 rows).
 constexpr int kShortRow = 28, kLongRow = 48, kParts = 8;
 template <int N>
 __device__ __forceinline__ void add_row(const double *val, const int32_t *col, const double *__restrict__ x, int k0, int k1, double (&part)[kParts]) {
@@ -145,9 +146,8 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) k_residual_noalloc(int
       }
       const int k0 = (int)((a < base ? base : a < base + m ? a : base + m) - base);
       const int k1 = (int)((z < base ? base : z < base + m ? z : base + m) - base);
-      const int kl = longrow ? k0 : k1;  // (nothing of a long row)
-      if (__any_sync(0xffffffffu, z - a > kShortRow && !longrow)) add_row<kParts>(sval[buf], scol[buf], x, k0, kl, part);
-      else add_row<4>(sval[buf], scol[buf], x, k0, kl, part);
+      if (z - a <= kShortRow) add_row<4>(sval[buf], scol[buf], x, k0, k1, part);
+      else if (!longrow) add_row<kParts>(sval[buf], scol[buf], x, k0, k1, part);
       for (unsigned of = __ballot_sync(0xffffffffu, longrow && k0 < k1); of; of &= of - 1) {
         const int l = __ffs(of) - 1, q0 = __shfl_sync(0xffffffffu, k0, l), q1 = __shfl_sync(0xffffffffu, k1, l);
         double p = 0.0;
