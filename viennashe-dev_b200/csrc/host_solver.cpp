@@ -1724,6 +1724,18 @@ void plan_sweep_tasks(const std::vector<System *> &sys, bool mixed, bool has_pc,
   plan_local_tasks(sys, mixed, P);
 }
 
+// Rows of an average level up to which a cluster of up to 8 CTAs factorises a system sooner than the whole
+// grid does.  ILU(0) and ILU(k) rows take 8 lanes, 512 of them at a time: us per level, cluster and grid,
+// 512 rows 3.9 and 6.8, 768 rows 6.2 and 5.7 (rows of 2 entries); 690 rows of a natural-order bar, first
+// order, 11.3 and 12.0, 907 rows 13.6 and 12.0.  ILUT rows take 128 threads, 32 of them at a time, and gain
+// over a warp of the grid what the lanes of a long row gain: 64 rows of 2 factor entries 8.2 and 9.8, 128
+// rows 15 and 9.5; 166 rows of 20 entries 57 and 166; 289 rows of 23 entries 84 and 87, 369 rows 100 and
+// 78; 102 rows of 60 entries 65 and 267; 565 rows of 9 entries 100 and 31.
+static double cluster_rows(const System &S) {
+  if (S.opts.precond != VSHE_PRECOND_ILUT) return 700;
+  return std::min(350.0, 50 + 10 * double(S.nnzL + S.nnzU) / double(std::max<int64_t>(S.n, 1)));
+}
+
 int Batch::build(Ctx &ctx, const std::vector<System *> &members) {
   int rc0 = 0;
   sys = members;
@@ -1785,11 +1797,10 @@ int Batch::build(Ctx &ctx, const std::vector<System *> &members) {
     slices(false, cptrU, csU, cqU, nlevU);
     // factorisation: merged level l = the forward-level-l rows of every member (all members,
     // whichever sweep they use)
-    // Members swept as one task whose levels hold up to 1024 rows on average are factorised by a
-    // cluster of CTAs each (k_ilu_cluster): the levels are short, so that the barrier after each sets the
-    // time, and it is cheaper the fewer CTAs it joins.
+    // Members swept as one task whose levels are short are factorised by a cluster of CTAs each
+    // (k_ilu_cluster): the barrier after each level sets the time, and it is cheaper the fewer CTAs it joins.
     std::vector<char> on_chain(size_t(nsys), 0);
-    for (int k = 0; k < nsys; ++k) on_chain[size_t(k)] = on_task[size_t(k)] == 1 && sys[size_t(k)]->n <= 1024 * int64_t(sys[size_t(k)]->nlevL);
+    for (int k = 0; k < nsys; ++k) on_chain[size_t(k)] = on_task[size_t(k)] == 1 && double(sys[size_t(k)]->n) <= cluster_rows(*sys[size_t(k)]) * sys[size_t(k)]->nlevL;
     nlevF = 0;
     for (int k = 0; k < nsys; ++k)
       if (!on_chain[size_t(k)]) nlevF = std::max(nlevF, sys[size_t(k)]->nlevL);
