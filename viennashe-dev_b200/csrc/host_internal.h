@@ -300,7 +300,6 @@ struct Ctx {
   // task sweep of one-CTA/cluster-per-task members: -1 autotuned per batch, 0 one CTA with staged
   // factor slices, K = 2, 4, 8 a cluster of K CTAs
   int task_sweep = -1;
-  void *pinned = nullptr;  // staging buffers of large downloads, from the first one on (copy_to_host)
   std::map<int64_t, std::unique_ptr<System>> systems;
   // vshe_solve_csr's pattern cache: the system of its last call (0 = none) and the options it was
   // created with (with copies of the option arrays)

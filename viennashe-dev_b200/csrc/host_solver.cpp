@@ -2641,7 +2641,6 @@ int vshe_destroy(vshe_ctx *ctx) {
   vshe::poisson_release_all(ctx);
   ctx->batches.clear();
   ctx->systems.clear();
-  if (ctx->pinned) cudaFreeHost(ctx->pinned);
   cudaStreamDestroy(ctx->stream);
   delete ctx;
   return VSHE_OK;

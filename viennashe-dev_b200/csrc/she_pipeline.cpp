@@ -8,13 +8,14 @@
 // viennashe::she::solve (viennashe/she/linear_solver.hpp:100-189).
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <map>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -440,63 +441,45 @@ void she_release_all(Ctx *ctx) {
 }
 }  // namespace vshe
 
-// Copies `bytes` of a device array that the context's stream has written to pageable host memory.  The
-// driver moves pageable memory through a pinned buffer with one thread, at 4.7 GB/s; large arrays
-// are split over kCopyThreads threads, each with two pinned buffers of its own (the context's, 16 MB in
-// all) and a stream, so that one buffer fills while the other is emptied.  The 262 MB of the bar 200 x 50 x
-// 160: 56 ms, now 23, and 36 the first time, of it the allocation of the buffers, for which smaller arrays do not
-// make up (24 MB: 3.1 ms, 4.1 and 27).
-constexpr size_t kCopyLarge = size_t(64) << 20, kCopyThreads = 4, kCopyBuffer = size_t(2) << 20;
+// Copies `bytes` of a device array that the context's stream has written to host memory.  Large arrays
+// are mostly fresh memory, whose page faults, taken one by one by the copying thread, cost more than the
+// copy.  So kCopyThreads threads fault the pages in, piece by piece, ahead of the copies; nothing is kept
+// between calls.  262 MB (x_full of the bar 200 x 50 x 160): fresh pages 57 ms, now 21, pages in use 16.1 and
+// 16.3; 94 MB 21 and 10, 5.5 and 5.9.  (Through pinned buffers and four copying threads 17.6 and 10.2 ms, but 11
+// more in the first call.)  Pinned, registered and managed memory has no such faults and takes one copy
+// (4.7 ms).
+constexpr size_t kCopyLarge = size_t(64) << 20, kCopyPiece = size_t(8) << 20;
+constexpr int kCopyThreads = 4;
 static cudaError_t copy_to_host(Ctx &ctx, void *dst, const void *src, size_t bytes) {
-  if (bytes >= kCopyLarge && !ctx.pinned && cudaHostAlloc(&ctx.pinned, 2 * kCopyThreads * kCopyBuffer, cudaHostAllocDefault) != cudaSuccess) {
-    ctx.pinned = nullptr;
-    (void)cudaGetLastError();
-  }
-  if (bytes < kCopyLarge || !ctx.pinned) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx.stream);
-  cudaError_t e = cudaStreamSynchronize(ctx.stream);
-  if (e != cudaSuccess) return e;
-  const size_t part = (bytes / kCopyThreads + 4095) & ~size_t(4095);
-  cudaError_t err[kCopyThreads];
-  auto copy = [&](size_t k) {
-    const size_t a = std::min(bytes, k * part), b = std::min(bytes, a + part), n = (b - a + kCopyBuffer - 1) / kCopyBuffer;
-    char *buf = (char *)ctx.pinned + 2 * k * kCopyBuffer;
-    cudaStream_t s = nullptr;
-    cudaEvent_t ev[2] = {nullptr, nullptr};
-    cudaError_t q = cudaSetDevice(ctx.device);
-    if (q == cudaSuccess) q = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-    for (int i = 0; i < 2 && q == cudaSuccess; ++i) q = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
-    for (size_t i = 0; i <= n && q == cudaSuccess; ++i) {
-      if (i < n) {
-        const size_t o = a + i * kCopyBuffer;
-        q = cudaMemcpyAsync(buf + (i & 1) * kCopyBuffer, (const char *)src + o, std::min(kCopyBuffer, b - o), cudaMemcpyDeviceToHost, s);
-        if (q == cudaSuccess) q = cudaEventRecord(ev[i & 1], s);
-      }
-      if (i > 0 && q == cudaSuccess && (q = cudaEventSynchronize(ev[(i - 1) & 1])) == cudaSuccess) {
-        const size_t o = a + (i - 1) * kCopyBuffer;
-        std::memcpy((char *)dst + o, buf + ((i - 1) & 1) * kCopyBuffer, std::min(kCopyBuffer, b - o));
-      }
+  cudaPointerAttributes at;
+  const bool pageable = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
+  (void)cudaGetLastError();
+  const size_t pieces = (bytes + kCopyPiece - 1) / kCopyPiece;
+  std::unique_ptr<std::atomic<bool>[]> ready(bytes >= kCopyLarge && pageable ? new (std::nothrow) std::atomic<bool>[pieces] : nullptr);
+  if (!ready) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx.stream);
+  for (size_t i = 0; i < pieces; ++i) ready[i].store(false, std::memory_order_relaxed);
+  std::atomic<size_t> next{0};
+  auto fault_in = [&]() {
+    for (size_t i; (i = next.fetch_add(1)) < pieces;) {
+      volatile char *a = (char *)dst + i * kCopyPiece, *b = (char *)dst + std::min(bytes, (i + 1) * kCopyPiece);
+      for (; a < b; a += 4096) *a = *a;
+      ready[i].store(true, std::memory_order_release);
     }
-    if (s) {
-      const cudaError_t w = cudaStreamSynchronize(s);  // no copy into the buffers stays behind
-      if (q == cudaSuccess) q = w;
-      cudaStreamDestroy(s);
-    }
-    for (cudaEvent_t v : ev)
-      if (v) cudaEventDestroy(v);
-    err[k] = q;
   };
   std::thread th[kCopyThreads];
-  size_t k = 1;
+  int started = 0;
   try {
-    for (; k < kCopyThreads; ++k) th[k] = std::thread(copy, k);
-  } catch (const std::system_error &) {  // no more threads: the rest here
+    for (; started < kCopyThreads; ++started) th[started] = std::thread(fault_in);
+  } catch (const std::exception &) {  // no more threads: those there are do it all, or none
   }
-  for (size_t j = k; j < kCopyThreads; ++j) copy(j);
-  copy(0);
-  for (size_t j = 1; j < k; ++j) th[j].join();
-  for (cudaError_t q : err)
-    if (q != cudaSuccess) return q;
-  return cudaSuccess;
+  cudaError_t e = cudaSuccess;
+  for (size_t i = 0; i < pieces && e == cudaSuccess; ++i) {
+    while (started && !ready[i].load(std::memory_order_acquire)) std::this_thread::yield();
+    const size_t o = i * kCopyPiece;
+    e = cudaMemcpyAsync((char *)dst + o, (const char *)src + o, std::min(kCopyPiece, bytes - o), cudaMemcpyDeviceToHost, ctx.stream);
+  }
+  for (int k = 0; k < started; ++k) th[k].join();
+  return e;
 }
 
 extern "C" {
