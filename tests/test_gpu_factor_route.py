@@ -13,6 +13,7 @@ pytestmark = pytest.mark.gpu
     (dict(precond="ilut", ilut_entries=60, ilut_drop=1e-7), 60, True), (dict(precond="ilut", ilut_entries=60, ilut_drop=1e-7), 400, False),
 ])
 def test_route(gpu_ctx, kw, rows, cluster):
+    import torch
     from torch.profiler import ProfilerActivity, profile
     rp, ci, v, _ = shapes._levels([rows] * 40)
     n = len(rp) - 1
@@ -20,6 +21,7 @@ def test_route(gpu_ctx, kw, rows, cluster):
     try:
         with profile(activities=[ProfilerActivity.CUDA]) as p:
             x, st = S.solve()
+            torch.cuda.synchronize()
     finally:
         S.free()
     assert st["status"] == 0

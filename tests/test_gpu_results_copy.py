@@ -23,6 +23,7 @@ def test_pageable_and_pinned():
         pinned = torch.empty(n, dtype=torch.float64).pin_memory()
         with profile(activities=[ProfilerActivity.CUDA]) as p:
             ctx._check(gpu._she_lib().vshe_she_results(ctx.h, P.h, C.cast(pinned.data_ptr(), C.POINTER(C.c_double)), None, None))
+            torch.cuda.synchronize()
         copies = sum(e.count for e in p.key_averages() if "DtoH" in e.key)
         x, _, _ = P.results()
         assert x.nbytes > 64 << 20 and np.any(x != 0.0)
