@@ -96,7 +96,6 @@ struct System {
   std::vector<int32_t> lgrp_lev, lgrp_blk, ugrp_lev, ugrp_blk;
   std::vector<int64_t> loff_h, uoff_h;    // SELL slot offsets of the L and U slices (host copies)
   std::vector<int64_t> lrow0_h, uslot0_h; // first solver row / slot of every L / U slice (host copies)
-  std::vector<int32_t> urow_h;            // solver row of every backward slot (host copy)
   int32_t nlevL = 0, nlevU = 0;
   int64_t nslA = 0, nslL = 0, nslU = 0;     // SELL slices
   int64_t padA = 0, padL = 0, padU = 0;     // SELL slots (incl. padding)
@@ -130,6 +129,13 @@ struct System {
   int32_t *d_stream_olds = nullptr;
   int64_t *d_stream_patch = nullptr;
   double *d_yslot = nullptr;
+  // The stream is a second copy of the factor that a sweep can do without (k_trsv_task): left out where
+  // the system would hold more than `room` bytes with it, and dropped when the context runs short
+  // (release_sweep_tables).
+  DevArena stream_arena;
+  size_t room = ~size_t(0);
+  size_t bytes() const { return arena.total + stream_arena.total; }
+  void drop_stream();
   int build_stream(Ctx &ctx, const Layout &Lt);
   int fill_stream(Ctx &ctx, bool all);
   int64_t tile_rows = 0;    // rows per reduction tile (0: not chosen yet; see Batch::autotune_tiles)
@@ -186,7 +192,7 @@ struct SweepPlan {
   // per member with local block tasks: the task numbers of its rows, by solver row
   std::vector<std::vector<int32_t>> lnum;
 };
-void plan_sweep_tasks(const std::vector<System *> &sys, bool mixed, bool has_pc, int64_t num_sms, SweepPlan &plan);
+void plan_sweep_tasks(const std::vector<System *> &sys, bool mixed, bool has_pc, int64_t num_sms, SweepPlan &plan, bool local = true);
 
 struct Batch {
   std::vector<System *> sys;
@@ -224,6 +230,13 @@ struct Batch {
     void *d_tasks = nullptr;
   } streams;
   std::vector<char> own_kernel;
+  // The records of the local tasks are a copy of the factor too: left out where the batch would hold more
+  // than `room` bytes with them, 0: not planned (a batch that never sweeps).  drop_tables: all tasks run
+  // the kernel above from then on; also before the stream of a member goes.
+  DevArena table_arena;
+  size_t room = ~size_t(0);
+  size_t bytes() const { return arena.total + tile_arena.total + table_arena.total; }
+  void drop_tables();
   int build_local(Ctx &ctx, const SweepPlan &plan);
   int fill_local(Ctx &ctx);
   bool use_local(const Ctx &ctx) const;
@@ -331,6 +344,13 @@ void she_release_all(Ctx *ctx);
 size_t she_bytes(Ctx *ctx);
 void poisson_release_all(Ctx *ctx);
 size_t poisson_bytes(Ctx *ctx);
+// Whether `bytes` more fit the context's budget, if need be without the streams and local tasks of its
+// systems and batches (they then sweep with k_trsv_task; the results do not change).
+bool fits_budget(Ctx *ctx, size_t bytes);
+size_t budget_left(Ctx *ctx);
+// drop the sweep tables of the context's SHE problems and of their batches, of its Poisson problems
+void she_release_tables(Ctx *ctx);
+void poisson_release_tables(Ctx *ctx);
 
 }  // namespace vshe
 

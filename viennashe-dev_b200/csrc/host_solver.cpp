@@ -989,7 +989,6 @@ void System::adopt_layout(const Layout &Lt) {
   lgrp_s0 = Lt.lgrp_s0; lgrp_lev = Lt.lgrp_lev; lgrp_blk = Lt.lgrp_blk;
   ugrp_s0 = Lt.ugrp_s0; ugrp_lev = Lt.ugrp_lev; ugrp_blk = Lt.ugrp_blk;
   loff_h = Lt.loff; uoff_h = Lt.uoff;
-  urow_h = Lt.urow;
   lrow0_h.assign(Lt.lstart.begin(), Lt.lstart.end()); uslot0_h.assign(Lt.ustart.begin(), Lt.ustart.end());
   nlevL = Lt.nlevL; nlevU = Lt.nlevU; nslA = Lt.nslA; nslL = Lt.nslL; nslU = Lt.nslU;
   padA = Lt.padA; padL = Lt.padL; padU = Lt.padU; nnzL = Lt.nnzL; nnzU = Lt.nnzU; nnzF = Lt.nnzF;
@@ -1110,13 +1109,17 @@ int System::build_stream(Ctx &ctx, const Layout &Lt) {
   const size_t chunks = put(stream.chunks.data(), sizeof(StreamChunk) * stream.chunks.size()), heads = put(stream.heads.data(), stream.heads.size()),
                recs = put(stream.recs.data(), sizeof(StreamRec) * stream.recs.size()), olds = put(stream.olds.data(), 4 * stream.olds.size()),
                patch = put(stream.patch.data(), 8 * stream.patch.size());
-  unsigned char *t = (unsigned char *)arena.alloc(up.size() + 256, e);
-  if (!t) return ctx.cuda_fail(e, "cudaMalloc stream tables");
-  if ((e = cudaMemcpyAsync(t, up.data(), up.size(), cudaMemcpyHostToDevice, ctx.stream)) != cudaSuccess) return ctx.cuda_fail(e, "upload stream tables");
   const size_t row = size_t(stream.ent_bytes + 255) & ~size_t(255), ys = (row + size_t(stream.row_bytes) + 255) & ~size_t(255),
                bytes = ys + sizeof(double) * size_t(n + kVecPad);
-  unsigned char *f = (unsigned char *)arena.alloc(bytes, e);
-  if (!f) return ctx.cuda_fail(e, "cudaMalloc stream");
+  unsigned char *t = nullptr, *f = nullptr;
+  if (arena.total + up.size() + 256 + bytes <= room && (t = (unsigned char *)stream_arena.alloc(up.size() + 256, e)))
+    f = (unsigned char *)stream_arena.alloc(bytes, e);
+  if (!f) {  // no room for it
+    (void)cudaGetLastError();
+    drop_stream();
+    return VSHE_OK;
+  }
+  if ((e = cudaMemcpyAsync(t, up.data(), up.size(), cudaMemcpyHostToDevice, ctx.stream)) != cudaSuccess) return ctx.cuda_fail(e, "upload stream tables");
   if ((e = cudaMemsetAsync(f + ys, 0, bytes - ys, ctx.stream)) != cudaSuccess) return ctx.cuda_fail(e, "memset");
   d_stream = (StreamChunk *)(t + chunks);
   d_stream_heads = t + heads;
@@ -1131,6 +1134,12 @@ int System::build_stream(Ctx &ctx, const Layout &Lt) {
   // (the upload's source goes with this call)
   if ((e = cudaStreamSynchronize(ctx.stream)) != cudaSuccess) return ctx.cuda_fail(e, "stream tables");
   return VSHE_OK;
+}
+
+void System::drop_stream() {
+  stream_arena.release();
+  stream = StreamPlan{};
+  d_stream = nullptr;
 }
 
 // all: the stream's tables (once); otherwise the factor's values (after every factorisation).
@@ -1279,7 +1288,7 @@ static void add_local_task(const std::vector<System *> &sys, int vb, SweepPlan &
 // One shape serves the batch: values for the largest local task; half as many warps again as an
 // average level has slices, since the slices' widths differ (bar 50 x 20 x 60, 5 slices: 9.8 us per
 // apply with 5 warps, 9.0 with 8, 9.1 with 10; bar 90 x 29 x 64, 14 slices: 97 with 12, 87 with 15).
-static void plan_local_tasks(const std::vector<System *> &sys, bool mixed, SweepPlan &P) {
+static void plan_local_tasks(const std::vector<System *> &sys, bool mixed, bool local, SweepPlan &P) {
   const int vb = mixed ? 4 : 8;
   const size_t nt = P.tasks.size();
   P.nrest = int(nt);
@@ -1313,7 +1322,7 @@ static void plan_local_tasks(const std::vector<System *> &sys, bool mixed, Sweep
   std::vector<char> kind(nt, 0);  // 0 neither, 1 local, 2 stream
   double slices = 0, levels = 0;
   int64_t most = 1;
-  bool fit = true;
+  bool fit = local;
   for (size_t t = 0; t < nt; ++t) {
     const Info &I = info[t];
     const size_t k = size_t(P.ctasks[t].sys);
@@ -1353,14 +1362,14 @@ static void plan_local_tasks(const std::vector<System *> &sys, bool mixed, Sweep
     L.rec0[k + 1] = int64_t(L.recs.size());
   }
   // most work first, as the plan lists them
-  std::vector<int64_t> work(L.tasks.size());
+  std::vector<int64_t> bytes(L.tasks.size());
   for (size_t t = 0; t < L.tasks.size(); ++t) {
     const size_t w0 = size_t(L.tasks[t].warp0), w1 = w0 + size_t(L.nwarp);
-    work[t] = (w1 < L.warps.size() ? L.warps[w1].off : L.bytes) - L.warps[w0].off;
+    bytes[t] = (w1 < L.warps.size() ? L.warps[w1].off : L.bytes) - L.warps[w0].off;
   }
   std::vector<size_t> by((size_t)L.tasks.size());
   std::iota(by.begin(), by.end(), size_t(0));
-  std::stable_sort(by.begin(), by.end(), [&](size_t x, size_t y) { return work[x] > work[y]; });
+  std::stable_sort(by.begin(), by.end(), [&](size_t x, size_t y) { return bytes[x] > bytes[y]; });
   std::vector<LocTask> sorted;
   for (size_t t : by) sorted.push_back(L.tasks[t]);
   L.tasks.swap(sorted);
@@ -1564,7 +1573,7 @@ void plan_stream(const System &S, const Layout &L, StreamPlan &P) {
 // bar: one CTA streams a task's factor and vectors at about kTaskBytesPerUs, and a level of the
 // grid-wide sweep costs about kGridLevelUs (its grid barrier and the latency of the level's
 // rows) on top of the apply's bytes at kGridBytesPerUs.
-void plan_sweep_tasks(const std::vector<System *> &sys, bool mixed, bool has_pc, int64_t num_sms_hint, SweepPlan &P) {
+void plan_sweep_tasks(const std::vector<System *> &sys, bool mixed, bool has_pc, int64_t num_sms_hint, SweepPlan &P, bool local) {
   const int nsys = int(sys.size());
   std::vector<char> &on_task = P.on_task;  // 0 grid, 1 whole system, 2 per block
   on_task.assign((size_t)nsys, 0);
@@ -1721,7 +1730,7 @@ void plan_sweep_tasks(const std::vector<System *> &sys, bool mixed, bool has_pc,
       P.has_tune_key = true;
     }
   }
-  plan_local_tasks(sys, mixed, P);
+  plan_local_tasks(sys, mixed, local, P);
 }
 
 // Rows of an average level up to which a cluster of up to 8 CTAs factorises a system sooner than the whole
@@ -1752,7 +1761,7 @@ int Batch::build(Ctx &ctx, const std::vector<System *> &members) {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
       num_sms = sms;
-    plan_sweep_tasks(sys, mixed, has_pc, num_sms, plan);
+    plan_sweep_tasks(sys, mixed, has_pc, num_sms, plan, room > 0);
   }
   const std::vector<char> &on_task = plan.on_task;
   const std::vector<TaskDev> &tasks = plan.tasks;
@@ -1948,47 +1957,19 @@ int Batch::build(Ctx &ctx, const std::vector<System *> &members) {
   ilu_grid = std::max(1, std::min(bpf, 4)) * num_sms;
   cudaError_t es = cudaStreamSynchronize(s);
   if (es != cudaSuccess) return ctx.cuda_fail(es, "batch upload");
-  if ((rc0 = build_local(ctx, plan))) return rc0;
-  return set_tiles(ctx);
+  if ((rc0 = set_tiles(ctx))) return rc0;
+  return build_local(ctx, plan);
 }
 
 bool Batch::use_local(const Ctx &ctx) const { return local.tasks + streams.tasks > 0 && ctx.task_sweep < 0; }
 
-// Device tables of the batch's local tasks (the plan's lists, and per member the slot of every row,
-// the columns in task numbers and the forward result by slot) and of its streams.
+// Device tables of the batch's local tasks (the plan's lists and the records, laid out here and filled by
+// fill_local) and of its streams.
 int Batch::build_local(Ctx &ctx, const SweepPlan &plan) {
   nrest = plan.nrest;
   own_kernel = plan.own_kernel;
-  cudaError_t e;
+  cudaError_t e = cudaSuccess;
   cudaStream_t s = ctx.stream;
-#define ALLOC(ptr, bytes)                                   \
-  ptr = arena.alloc(size_t(bytes), e);                      \
-  if (!ptr) return ctx.cuda_fail(e, "cudaMalloc batch " #ptr);
-#define TABLE(dst, vec)                                                                                                       \
-  ALLOC(dst, std::max<size_t>(sizeof(vec[0]) * vec.size(), 16));                                                                \
-  if (!vec.empty() && (e = cudaMemcpyAsync(dst, vec.data(), sizeof(vec[0]) * vec.size(), cudaMemcpyHostToDevice, s)) != cudaSuccess) \
-    return ctx.cuda_fail(e, "upload batch " #dst);
-  const LocalPlan &L = plan.local;
-  if (plan.nlocal) {
-    local.tasks = plan.nlocal;
-    local.nwarp = L.nwarp; local.ring = L.ring; local.slots = L.slots; local.slot_bytes = L.slot_bytes;
-    local.rec0 = L.rec0;
-    TABLE(local.d_tasks, L.tasks);
-    TABLE(local.d_warps, L.warps);
-    TABLE(local.d_recs, L.recs);
-    ALLOC(local.d_buf, L.bytes);
-    TABLE(local.d_runs, L.runs);
-    for (size_t k = 0; k < sys.size(); ++k) {
-      if (plan.lnum[k].empty()) continue;
-      void *num;
-      TABLE(num, plan.lnum[k]);
-      std::vector<char> sd(vk_sysdev_size());
-      sys[k]->fill_sysdev(sd.data());
-      const int rc = vk_local_fill(mixed ? 1 : 0, sd.data(), int(L.rec0[k + 1] - L.rec0[k]), (const LocRec *)local.d_recs + L.rec0[k],
-                                   (const int32_t *)num, L.ring, 1, local.d_buf, s);
-      if (rc) return ctx.cuda_fail(cudaError_t(rc), "local sweep records");
-    }
-  }
   std::vector<StreamTask> st;
   for (size_t t = size_t(plan.nrest + plan.nlocal); t < plan.tasks.size(); ++t) {
     const int32_t k = plan.tasks[t].sys;
@@ -2004,12 +1985,59 @@ int Batch::build_local(Ctx &ctx, const SweepPlan &plan) {
     streams.nwarp = std::max(streams.nwarp, Q.nwarp);
     streams.smem = std::max(streams.smem, int(local_smem_bytes(Q.ring, Q.stage)));
   }
+  const LocalPlan &L = plan.local;
+  size_t total = size_t(plan.nlocal ? L.bytes : 0);
+  auto bytes = [](const auto &v) { return std::max<size_t>(sizeof(v[0]) * v.size(), 16); };
+  total += bytes(L.tasks) + bytes(L.warps) + bytes(L.recs) + bytes(L.runs) + bytes(st);
+  for (const std::vector<int32_t> &num : plan.lnum) total += 4 * num.size();
+  if (this->bytes() + total > room) { drop_tables(); return VSHE_OK; }
+  bool fit = true;
+  auto table = [&](const auto &v) -> void * {
+    void *d = fit ? table_arena.alloc(bytes(v), e) : nullptr;
+    if (!d) { fit = false; return nullptr; }
+    if (!v.empty() && e == cudaSuccess) e = cudaMemcpyAsync(d, v.data(), sizeof(v[0]) * v.size(), cudaMemcpyHostToDevice, s);
+    return d;
+  };
+  std::vector<void *> num(sys.size(), nullptr);
+  if (plan.nlocal) {
+    local.tasks = plan.nlocal;
+    local.nwarp = L.nwarp; local.ring = L.ring; local.slots = L.slots; local.slot_bytes = L.slot_bytes;
+    local.rec0 = L.rec0;
+    local.d_tasks = table(L.tasks);
+    local.d_warps = table(L.warps);
+    local.d_recs = table(L.recs);
+    local.d_runs = table(L.runs);
+    for (size_t k = 0; k < sys.size(); ++k)
+      if (!plan.lnum[k].empty()) num[k] = table(plan.lnum[k]);
+    if (fit && !(local.d_buf = table_arena.alloc(size_t(L.bytes), e))) fit = false;
+  }
   streams.tasks = int(st.size());
-  if (streams.tasks) { TABLE(streams.d_tasks, st); }
-#undef ALLOC
-#undef TABLE
-  if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return ctx.cuda_fail(e, "local sweep tables");
-  return VSHE_OK;
+  if (streams.tasks) streams.d_tasks = table(st);
+  if (!fit) {  // no memory for them: every task runs k_trsv_task or k_trsv_cluster
+    (void)cudaGetLastError();
+    cudaStreamSynchronize(s);
+    drop_tables();
+    return VSHE_OK;
+  }
+  for (size_t k = 0; k < sys.size() && e == cudaSuccess; ++k) {
+    if (!num[k]) continue;
+    std::vector<char> sd(vk_sysdev_size());
+    sys[k]->fill_sysdev(sd.data());
+    e = cudaError_t(vk_local_fill(mixed ? 1 : 0, sd.data(), int(L.rec0[k + 1] - L.rec0[k]), (const LocRec *)local.d_recs + L.rec0[k],
+                                  (const int32_t *)num[k], L.ring, 1, local.d_buf, s));
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  return e == cudaSuccess ? VSHE_OK : ctx.cuda_fail(e, "local sweep tables");
+}
+
+void Batch::drop_tables() {
+  table_arena.release();
+  local = LocalTables{};
+  streams = StreamTables{};
+  nrest = ntasks;
+  own_kernel.assign(size_t(nsys), 0);
+  tasks_tuned = false;
+  if (chunk_exec) { cudaGraphExecDestroy(chunk_exec); chunk_exec = nullptr; }
 }
 
 // The members' present factors into the local tasks' records: after a factorisation, and before the
@@ -2576,7 +2604,7 @@ int Batch::solve(Ctx &ctx, std::vector<vshe_solve_stats> &stats) {
     st.solve_ms = ms_solve;
     st.levels_L = S->nlevL;
     st.levels_U = S->nlevU;
-    st.bytes_device = int64_t(S->arena.total);
+    st.bytes_device = int64_t(S->bytes());
     const int tk = task_kind.empty() ? 0 : task_kind[size_t(k)];
     st.sweep_ctas = !has_pc ? 0 : tk ? (task_kernel > 0 && !(use_local(ctx) && own_kernel[size_t(k)]) ? task_kernel : 1) : trsv_grid;
     st.sweep_mode = !has_pc ? 0
@@ -2591,6 +2619,21 @@ int Batch::solve(Ctx &ctx, std::vector<vshe_solve_stats> &stats) {
     st.status = code;
   }
   return VSHE_OK;
+}
+
+size_t budget_left(Ctx *ctx) {
+  const size_t used = vshe_bytes_in_use((vshe_ctx *)ctx);
+  return used < ctx->budget ? ctx->budget - used : 0;
+}
+
+bool fits_budget(Ctx *ctx, size_t bytes) {
+  if (bytes <= budget_left(ctx)) return true;
+  cudaStreamSynchronize(ctx->stream);
+  for (auto &kv : ctx->batches) kv.second->drop_tables();
+  for (auto &kv : ctx->systems) kv.second->drop_stream();
+  she_release_tables(ctx);
+  poisson_release_tables(ctx);
+  return bytes <= budget_left(ctx);
 }
 
 }  // namespace vshe
@@ -2651,8 +2694,8 @@ const char *vshe_last_error(vshe_ctx *ctx) { return ctx ? ctx->last_error.c_str(
 size_t vshe_bytes_in_use(vshe_ctx *ctx) {
   if (!ctx) return 0;
   size_t t = 0;
-  for (auto &kv : ctx->systems) t += kv.second->arena.total;
-  for (auto &kv : ctx->batches) t += kv.second->arena.total + kv.second->tile_arena.total;
+  for (auto &kv : ctx->systems) t += kv.second->bytes();
+  for (auto &kv : ctx->batches) t += kv.second->bytes();
   return t + vshe::she_bytes(ctx) + vshe::poisson_bytes(ctx);
 }
 
@@ -2715,8 +2758,9 @@ int vshe_system_create(vshe_ctx *ctx, int64_t n, int64_t nnz, const int64_t *rp,
   if (opts) o = *opts; else vshe_default_opts(&o);
   // admission against the HBM budget (upper estimate of the system's footprint)
   const size_t est = size_t(nnz) * (4 + 8 + 8 + 4 + 8 + 8 + 8 + 8) + size_t(n) * (8 * 8 + 9 * 8 + 32);
-  if (vshe_bytes_in_use(ctx) + est > ctx->budget) return ctx->fail(VSHE_E_BUDGET, std::to_string(est) + " bytes requested");
+  if (!fits_budget(ctx, est)) return ctx->fail(VSHE_E_BUDGET, std::to_string(est) + " bytes requested");
   std::unique_ptr<System> S(new System);
+  S->room = budget_left(ctx);
   int rc = S->create(*ctx, n, nnz, rp, ci, v, rhs, o);
   if (rc) return rc;
   S->opts.block_ptr = nullptr;  // read during creation only
@@ -2747,6 +2791,7 @@ static Batch *get_batch(vshe_ctx *ctx, const std::vector<int64_t> &hs, int &rc) 
     mem.push_back(f->second.get());
   }
   std::unique_ptr<Batch> B(new Batch);
+  B->room = budget_left(ctx);
   rc = B->build(*ctx, mem);
   if (rc) return nullptr;
   Batch *p = B.get();

@@ -35,8 +35,8 @@ struct PoissonProblem {
   bool assembled = false;
   size_t bytes() const {
     size_t t = arena.total;
-    if (sys) t += sys->arena.total;
-    if (batch) t += batch->arena.total + batch->tile_arena.total;
+    if (sys) t += sys->bytes();
+    if (batch) t += batch->bytes();
     return t;
   }
 };
@@ -51,6 +51,16 @@ size_t poisson_bytes(Ctx *ctx) {
   if (it != g_poi.end())
     for (auto &kv : it->second) t += kv.second->bytes();
   return t;
+}
+
+void poisson_release_tables(Ctx *ctx) {
+  std::lock_guard<std::mutex> lk(g_poi_mu);
+  auto it = g_poi.find(ctx);
+  if (it == g_poi.end()) return;
+  for (auto &kv : it->second) {
+    if (kv.second->batch) kv.second->batch->drop_tables();
+    if (kv.second->sys) kv.second->sys->drop_stream();
+  }
 }
 
 void poisson_release_all(Ctx *ctx) {
@@ -147,7 +157,7 @@ int vshe_poisson_create(vshe_ctx *ctx, const vshe_device_desc *d, const double *
   // admission against the context's budget (a bound of the tables below and of the solver)
   const size_t est = size_t(nc) * 128 + size_t(nf) * 64 + size_t(cfp[nc]) * 12 +
                      size_t(nnz) * (4 + 8 + 8 + 4 + 8 + 8 + 8 + 8) + size_t(nu) * (8 * 8 + 9 * 8 + 32) + (size_t(1) << 20);
-  if (vshe_bytes_in_use(ctx) + est > ctx->budget) return ctx->fail(VSHE_E_BUDGET, std::to_string(est) + " bytes requested");
+  if (!fits_budget(ctx, est)) return ctx->fail(VSHE_E_BUDGET, std::to_string(est) + " bytes requested");
   int rc = VSHE_OK;
   DevArena &ar = Q->arena;
   PoissonDev &P = Q->P;
@@ -193,11 +203,13 @@ int vshe_poisson_create(vshe_ctx *ctx, const vshe_device_desc *d, const double *
     }
     o.precision = VSHE_PRECISION_FP64;
     Q->sys.reset(new System);
+    Q->sys->room = budget_left(ctx) - std::min(budget_left(ctx), Q->bytes());
     rc = Q->sys->create_borrowed(*ctx, nu, nnz, Q->rp.data(), Q->ci.data(), Q->d_rp, Q->d_ci, Q->d_val, Q->d_rhs, o, nullptr);
     if (rc) return rc;
     Q->sys->opts.block_ptr = nullptr;
     Q->sys->opts.perm = nullptr;
     Q->batch.reset(new Batch);
+    Q->batch->room = budget_left(ctx) - std::min(budget_left(ctx), Q->bytes());
     std::vector<System *> mem{Q->sys.get()};
     if ((rc = Q->batch->build(*ctx, mem))) return rc;
   }

@@ -67,7 +67,7 @@ struct SheProblem {
   int create_device(Ctx &ctx);  // = create_device_pattern, build_layout, create_device_finish
   int create_device_pattern(Ctx &ctx);
   void build_layout();
-  int create_device_finish(Ctx &ctx);
+  int create_device_finish(Ctx &ctx, bool alone = true);  // alone: its own batch will sweep
   int symbolic_full(Ctx &ctx);
   int fill_full(Ctx &ctx);
   int assemble(Ctx &ctx, int upto);
@@ -321,8 +321,11 @@ void SheProblem::build_layout() {
 }
 
 // Device buffers of the reduced system from the layout, and the problem's own batch.
-int SheProblem::create_device_finish(Ctx &ctx) {
+int SheProblem::create_device_finish(Ctx &ctx, bool alone) {
   if (!layout_) return ctx.fail(VSHE_E_INVALID_ARGUMENT, "layout not built");
+  // the sweeps' own tables stay within the bound the problem was admitted with
+  const size_t most = estimate_bytes();
+  sys->room = most - std::min(most, arena.total);
   int rc = layout_rc_ ? ctx.fail(layout_rc_, layout_err_) : sys->setup_from_layout(ctx, *layout_);
   layout_.reset();
   std::vector<double>().swap(hval_);
@@ -330,7 +333,9 @@ int SheProblem::create_device_finish(Ctx &ctx) {
   sys->opts.block_ptr = nullptr;  // the pointers above are only read during creation
   sys->opts.perm = nullptr;
   std::vector<int32_t>().swap(node_perm_);
+  const size_t held = arena.total + sys->bytes();
   batch.reset(new Batch);
+  batch->room = alone ? most - std::min(most, held) : 0;
   std::vector<System *> mem{sys.get()};
   return batch->build(ctx, mem);
 }
@@ -411,8 +416,8 @@ static std::mutex g_she_mu;
 
 static size_t problem_bytes(const SheProblem *S) {
   size_t b = S->arena.total;
-  if (S->sys) b += S->sys->arena.total;
-  if (S->batch) b += S->batch->arena.total + S->batch->tile_arena.total;
+  if (S->sys) b += S->sys->bytes();
+  if (S->batch) b += S->batch->bytes();
   return b;
 }
 
@@ -422,6 +427,9 @@ size_t vshe::she_bytes(Ctx *ctx) {
   auto it = g_she.find(ctx);
   if (it != g_she.end())
     for (auto &kv : it->second) t += problem_bytes(kv.second.get());
+  auto bt = g_she_batches.find(ctx);
+  if (bt != g_she_batches.end())
+    for (auto &kv : bt->second) t += kv.second->table_arena.total;
   return t;
 }
 
@@ -434,6 +442,18 @@ static SheProblem *find_she(vshe_ctx *ctx, int64_t h) {
 }
 
 namespace vshe {
+void she_release_tables(Ctx *ctx) {
+  std::lock_guard<std::mutex> lk(g_she_mu);
+  auto bt = g_she_batches.find(ctx);
+  if (bt != g_she_batches.end())
+    for (auto &kv : bt->second) kv.second->drop_tables();
+  auto it = g_she.find(ctx);
+  if (it == g_she.end()) return;
+  for (auto &kv : it->second) {
+    if (kv.second->batch) kv.second->batch->drop_tables();
+    if (kv.second->sys) kv.second->sys->drop_stream();
+  }
+}
 void she_release_all(Ctx *ctx) {
   std::lock_guard<std::mutex> lk(g_she_mu);
   g_she_batches.erase(ctx);
@@ -502,7 +522,7 @@ int vshe_she_create(vshe_ctx *ctx, const vshe_device_desc *d, const vshe_she_con
   if (rc) return rc;
   // admission against the context's HBM budget before any allocation
   const size_t est = S->estimate_bytes();
-  if (vshe_bytes_in_use(ctx) + est > ctx->budget) return ctx->fail(VSHE_E_BUDGET, std::to_string(est) + " bytes (upper bound) requested");
+  if (!fits_budget(ctx, est)) return ctx->fail(VSHE_E_BUDGET, std::to_string(est) + " bytes (upper bound) requested");
   rc = S->create_device(*ctx);
   if (rc) return rc;
   int64_t h = ++ctx->next_handle;
@@ -579,7 +599,7 @@ int vshe_she_info_get(vshe_ctx *ctx, int64_t h, vshe_she_info *info) {
   info->n_facets = S->H.nf;
   info->n_contacts = S->ncontacts;
   info->hbar_omega = S->H.hbar_omega;
-  info->bytes_device = int64_t(S->arena.total + (S->sys ? S->sys->arena.total : 0) + (S->batch ? S->batch->arena.total + S->batch->tile_arena.total : 0));
+  info->bytes_device = int64_t(problem_bytes(S));
   info->levels_L = S->sys ? S->sys->nlevL : 0;
   info->levels_U = S->sys ? S->sys->nlevU : 0;
   info->nnz_factor = S->sys ? S->sys->nnzL + S->sys->nnzU : 0;
@@ -764,6 +784,7 @@ int vshe_she_run_batch(vshe_ctx *ctx, int32_t count, const int64_t *handles, vsh
     std::vector<System *> mem;
     for (SheProblem *S : probs) mem.push_back(S->sys.get());
     std::unique_ptr<Batch> nb(new Batch);
+    nb->room = budget_left(ctx);
     int rc = nb->build(*ctx, mem);
     if (rc) return rc;
     B = nb.get();
@@ -906,7 +927,7 @@ constexpr int64_t kAsyncLayoutRows = int64_t(1) << 18;
 int Server::finish_setup(ServeRequest *r) {
   Ctx &c = *ctx;
   SheProblem *S = r->prob.get();
-  int rc = S->create_device_finish(c);
+  int rc = S->create_device_finish(c, false);
   if (!rc) rc = S->assemble(c, 3);
   if (!rc) {
     S->sys->prepare(c);
@@ -932,8 +953,12 @@ void Server::end_setting_up(int status) {
 
 int Server::admit(std::vector<ServeRequest *> &fresh) {
   Ctx &c = *ctx;
-  size_t held = 0;
-  for (ServeRequest *r : active) held += problem_bytes(r->prob.get());
+  // held: what the requests cannot do without; tables: the sweeps' own, given up before a request has to wait
+  size_t held = 0, tables = batch ? batch->table_arena.total : 0;
+  for (ServeRequest *r : active) {
+    held += problem_bytes(r->prob.get()) - r->prob->sys->stream_arena.total;
+    tables += r->prob->sys->stream_arena.total;
+  }
   for (ServeRequest *r : setting_up) held += r->need;
   // requests whose layout has finished
   for (auto it = setting_up.begin(); it != setting_up.end();) {
@@ -970,6 +995,11 @@ int Server::admit(std::vector<ServeRequest *> &fresh) {
     }
     r->t_admit = std::chrono::steady_clock::now();
     if (!rc && held + need > opts.hbm_budget) rc = c.fail(VSHE_E_BUDGET, "request alone exceeds the server's HBM budget");
+    if (!rc && tables && held + tables + need > opts.hbm_budget) {
+      if (batch) batch->drop_tables();
+      for (ServeRequest *q : active) q->prob->sys->drop_stream();
+      tables = 0;
+    }
     if (!rc) rc = S->create_device_pattern(c);
     if (rc) { r->res.status = rc; complete(r, rc); continue; }
     r->prob = std::move(S);
@@ -1015,7 +1045,13 @@ int Server::step() {
     if (active.empty()) return VSHE_OK;
     std::vector<System *> mem;
     for (ServeRequest *r : active) mem.push_back(r->prob->sys.get());
+    // (the batch before goes first: two of them need not fit)
+    batch.reset();
+    size_t held = 0;
+    for (ServeRequest *r : active) held += problem_bytes(r->prob.get());
+    for (ServeRequest *r : setting_up) held += r->need;
     std::unique_ptr<Batch> nb(new Batch);
+    nb->room = std::max(opts.hbm_budget, held) - held;
     if ((rc = nb->build(c, mem))) return rc;
     batch = std::move(nb);
     // carry the running members' states over; start the newcomers
