@@ -182,8 +182,7 @@ struct SweepPlan {
   std::vector<SliceDesc> sdesc;
   std::vector<ClusterTask> ctasks;
   std::vector<int64_t> clv;
-  int64_t tune_key_tasks = 0;
-  bool has_tune_key = false;
+  std::vector<int64_t> work;     // of each task, as `tasks`
   // `tasks` in this order: those of k_trsv_task or k_trsv_cluster, local ones (k_trsv_local), streams
   // (k_trsv_stream)
   int nrest = 0, nlocal = 0;
@@ -214,7 +213,8 @@ struct Batch {
   int64_t *d_clv = nullptr;
   int task_kernel = 4;                 // 0 staged single CTA per task, K > 0 cluster of K CTAs per task
   bool tasks_tuned = false;
-  int64_t tune_key_tasks = -1, tune_key_grid = -1;  // shape classes of the task and grid-wide sweeps
+  // shape classes of the task sweep (the tasks [0, nrest), all tasks) and of the grid-wide sweep
+  int64_t tune_key_tasks = -1, tune_key_all = -1, tune_key_grid = -1;
   std::vector<double> task_tune_ms;    // ms per apply: staged, clusters of 2, 4, 8
   // tasks [0, nrest) run the kernel above; the others are local tasks (trsv_local.cu) and
   // streams (trsv_stream.cu) unless vshe_set_task_sweep names a kernel for all

@@ -1338,13 +1338,15 @@ static void plan_local_tasks(const std::vector<System *> &sys, bool mixed, bool 
   std::vector<TaskDev> tk;
   std::vector<ClusterTask> ct;
   std::vector<size_t> order;
+  std::vector<int64_t> work;
   for (int part = 0; part < 3; ++part)
     for (size_t t = 0; t < nt; ++t)
-      if (kind[t] == part) { tk.push_back(P.tasks[t]); ct.push_back(P.ctasks[t]); order.push_back(t); }
+      if (kind[t] == part) { tk.push_back(P.tasks[t]); ct.push_back(P.ctasks[t]); order.push_back(t); work.push_back(P.work[t]); }
   P.nrest = int(std::count(kind.begin(), kind.end(), 0));
   P.nlocal = int(std::count(kind.begin(), kind.end(), 1));
   P.tasks.swap(tk);
   P.ctasks.swap(ct);
+  P.work.swap(work);
   std::fill(P.own_kernel.begin(), P.own_kernel.end(), 1);
   for (int t = 0; t < P.nrest; ++t) P.own_kernel[size_t(P.ctasks[size_t(t)].sys)] = 0;
   L.rec0.assign(sys.size() + 1, 0);
@@ -1721,14 +1723,8 @@ void plan_sweep_tasks(const std::vector<System *> &sys, bool mixed, bool has_pc,
       t.second.pad = 0;
       tasks.push_back(t.second);
     }
-    const int ntasks = int(tasks.size());
-    // shape class of the task sweep: precision, the largest task's work and the task count (the
-    // apply's time is the largest task's walk, in waves of one CTA per SM)
-    auto log2c = [](int64_t v) { int c = 0; while (v > 1) { v >>= 1; ++c; } return c; };
-    if (!tw.empty()) {
-      P.tune_key_tasks = (int64_t(mixed ? 1 : 0) << 40) | (int64_t(log2c(tw.front().first)) << 20) | int64_t(log2c(ntasks));
-      P.has_tune_key = true;
-    }
+    P.work.clear();
+    for (auto &t : tw) P.work.push_back(t.first);
   }
   plan_local_tasks(sys, mixed, local, P);
 }
@@ -1770,7 +1766,16 @@ int Batch::build(Ctx &ctx, const std::vector<System *> &members) {
   const std::vector<ClusterTask> &ctasks = plan.ctasks;
   const std::vector<int64_t> &clv = plan.clv;
   ntasks = int(tasks.size());
-  if (plan.has_tune_key) tune_key_tasks = plan.tune_key_tasks;
+  // shape class of the task sweep: precision, the largest task's work and the task count (the apply's time
+  // is the largest task's walk, in waves of one CTA per SM), of the tasks that are left to it
+  auto task_key = [&](size_t count) {
+    auto log2c = [](int64_t v) { int c = 0; while (v > 1) { v >>= 1; ++c; } return c; };
+    if (count == 0) return int64_t(-1);
+    const int64_t most = *std::max_element(plan.work.begin(), plan.work.begin() + int64_t(count));
+    return (int64_t(mixed ? 1 : 0) << 40) | (int64_t(log2c(most)) << 20) | int64_t(log2c(int64_t(count)));
+  };
+  tune_key_tasks = task_key(size_t(plan.nrest));
+  tune_key_all = task_key(size_t(ntasks));
   grid_group = false;
   {
     int64_t grid_rows = 0;
@@ -2035,6 +2040,7 @@ void Batch::drop_tables() {
   local = LocalTables{};
   streams = StreamTables{};
   nrest = ntasks;
+  tune_key_tasks = tune_key_all;
   own_kernel.assign(size_t(nsys), 0);
   tasks_tuned = false;
   if (chunk_exec) { cudaGraphExecDestroy(chunk_exec); chunk_exec = nullptr; }
