@@ -242,7 +242,10 @@ struct Batch {
   bool use_local(const Ctx &ctx) const;
   bool local_captured = false;  // use_local when the chunk's graph was captured
   int launch_tasks(Ctx &ctx, int which);
-  int launch_task_kernel(Ctx &ctx, int count, int which);
+  int launch_task_kernel(Ctx &ctx, int count, int which, cudaStream_t s);
+  // the stream of k_trsv_stream beside the other tasks of a batch of both kinds, its start and its end
+  cudaStream_t side = nullptr;
+  cudaEvent_t side_event[2] = {nullptr, nullptr};
   int autotune_tasks(Ctx &ctx);
   bool grid_group = true;
   // the BiCGStab iteration chunk (check_every iterations) captured once as a CUDA graph and
@@ -251,7 +254,7 @@ struct Batch {
   int chunk_every = 0;
   long long chunk_launches = 0;
   bool graph_failed = false;
-  ~Batch() { if (chunk_exec) cudaGraphExecDestroy(chunk_exec); }
+  ~Batch();
   // row tiles: every member's own tile_rows rows per tile, rebuilt by set_tiles
   DevArena tile_arena;
   DevArena arena;

@@ -2024,6 +2024,11 @@ int Batch::build_local(Ctx &ctx, const SweepPlan &plan) {
     drop_tables();
     return VSHE_OK;
   }
+  if (nrest + local.tasks > 0 && streams.tasks > 0 && e == cudaSuccess) {
+    for (cudaEvent_t &v : side_event)
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+  }
   for (size_t k = 0; k < sys.size() && e == cudaSuccess; ++k) {
     if (!num[k]) continue;
     std::vector<char> sd(vk_sysdev_size());
@@ -2033,6 +2038,13 @@ int Batch::build_local(Ctx &ctx, const SweepPlan &plan) {
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   return e == cudaSuccess ? VSHE_OK : ctx.cuda_fail(e, "local sweep tables");
+}
+
+Batch::~Batch() {
+  if (chunk_exec) cudaGraphExecDestroy(chunk_exec);
+  for (cudaEvent_t v : side_event)
+    if (v) cudaEventDestroy(v);
+  if (side) cudaStreamDestroy(side);
 }
 
 void Batch::drop_tables() {
@@ -2195,26 +2207,37 @@ int Batch::factor(Ctx &ctx) {
 // k_trsv_stream (unless vshe_set_task_sweep names a kernel), the others with task_kernel: 0 = one
 // CTA per task with the factor slices staged through shared memory (k_trsv_task), K > 0 = one
 // thread-block cluster of K CTAs per task (k_trsv_cluster).
+//
+// Streams and block tasks (a batch's are local all or none) run side by side, the streams on a stream of
+// the batch that starts after the context's and that the context's waits for.  us per apply, FP64
+// factors, all tasks in k_trsv_task, one kernel after the other, and now: diode of 50 boxes and bar 160 x
+// 40 x 100, third order, 469, 519 and 291; diode of 100 boxes and the same bar 845, 801 and 577; FP32 factors,
+// 250-box diode, first order, and bar 120 x 30 x 70, third order, 590, 216 and 123.
 int Batch::launch_tasks(Ctx &ctx, int which) {
   cudaStream_t s = ctx.stream;
-  int count = ntasks;
-  if (use_local(ctx)) {
-    int rc = 0;
-    if (streams.tasks)
-      rc = vk_trsv_stream(mixed ? 1 : 0, streams.tasks, streams.nwarp, streams.smem, d_sysdev, d_state, d_active, streams.d_tasks, which, d_bar,
-                          d_err, s);
-    if (!rc && local.tasks)
-      rc = vk_trsv_local(mixed ? 1 : 0, local.tasks, local.nwarp, local.ring, local.slots, local.slot_bytes, d_sysdev, d_state,
-                         d_active, local.d_tasks, local.d_runs, local.d_warps, local.d_buf, which, d_bar, d_err, s);
-    if (rc) return rc;
-    count = nrest;
+  if (!use_local(ctx)) return launch_task_kernel(ctx, ntasks, which, s);
+  const bool both = side != nullptr;
+  if (both) {
+    cudaEventRecord(side_event[0], s);
+    cudaStreamWaitEvent(side, side_event[0], 0);
   }
-  return count ? launch_task_kernel(ctx, count, which) : 0;
+  int rc = 0;
+  if (nrest) rc = launch_task_kernel(ctx, nrest, which, s);
+  if (!rc && local.tasks)
+    rc = vk_trsv_local(mixed ? 1 : 0, local.tasks, local.nwarp, local.ring, local.slots, local.slot_bytes, d_sysdev, d_state, d_active,
+                       local.d_tasks, local.d_runs, local.d_warps, local.d_buf, which, d_bar, d_err, s);
+  if (!rc && streams.tasks)
+    rc = vk_trsv_stream(mixed ? 1 : 0, streams.tasks, streams.nwarp, streams.smem, d_sysdev, d_state, d_active, streams.d_tasks, which, d_bar,
+                        d_err, both ? side : s);
+  if (both) {
+    cudaEventRecord(side_event[1], side);
+    cudaStreamWaitEvent(s, side_event[1], 0);
+  }
+  return rc;
 }
 
 // the first `count` tasks with k_trsv_task or k_trsv_cluster
-int Batch::launch_task_kernel(Ctx &ctx, int count, int which) {
-  cudaStream_t s = ctx.stream;
+int Batch::launch_task_kernel(Ctx &ctx, int count, int which, cudaStream_t s) {
   if (task_kernel == 0)
     return mixed ? vk_trsv_task_f32(count, d_sysdev, d_state, d_active, d_tasks, d_chunks, d_sdesc, which, d_bar, d_err, s)
                  : vk_trsv_task_f64(count, d_sysdev, d_state, d_active, d_tasks, d_chunks, d_sdesc, which, d_bar, d_err, s);
@@ -2255,9 +2278,9 @@ int Batch::autotune_tasks(Ctx &ctx) {
   task_tune_ms.clear();
   for (int k : {0, 2, 4, 8}) {
     task_kernel = k;
-    int rc = launch_task_kernel(ctx, nrest, 0);  // warm-up
+    int rc = launch_task_kernel(ctx, nrest, 0, s);  // warm-up
     cudaEventRecord(a, s);
-    for (int r = 0; r < 3; ++r) rc |= launch_task_kernel(ctx, nrest, 0);
+    for (int r = 0; r < 3; ++r) rc |= launch_task_kernel(ctx, nrest, 0, s);
     cudaEventRecord(b, s);
     cudaError_t e = cudaEventSynchronize(b);
     if (rc || e != cudaSuccess) { cudaEventDestroy(a); cudaEventDestroy(b); return ctx.cuda_fail(e != cudaSuccess ? e : cudaError_t(rc), "autotune task sweeps"); }
