@@ -45,8 +45,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, unsign
   return true;
 }
 // The same for a whole warp, whose lanes all learn the same outcome: what follows a failed wait (barriers
-// of the CTA, warp-wide instructions) must not find the warp split.
+// of the CTA, warp-wide instructions) must not find the warp split.  (One poll and a vote first, the loop
+// out of the way: the local sweeps take 0.4 % longer than with lanes that decide alone, with a vote after
+// the loop 2.8 %.)
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, unsigned parity, unsigned long long limit, int32_t *err) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit, err));
 }
 // Waits for a phase regardless of the error word, at most kDrainPolls polls: copies in flight
