@@ -160,10 +160,6 @@ struct System {
   void fill_sysdev(void *out) const;
 };
 
-// Several systems solved together.
-// Sweep plan of a batch: per member 0 (grid-wide sweep), 1 (one task for the system) or 2 (tasks of
-// preconditioner blocks); the tasks, the chunks of their levels, the chunks' slice descriptors,
-// and the level slice ranges of the cluster sweeps.
 // Local tasks of a batch (k_trsv_local): the tables the kernel reads, every member's records (member k:
 // recs [rec0[k], rec0[k + 1])), the records' size and the launch shape.
 struct LocalPlan {
@@ -173,8 +169,11 @@ struct LocalPlan {
   std::vector<LocRec> recs;
   std::vector<int64_t> rec0;
   int64_t bytes = 0;
-  int nwarp = 0, ring = 0, slots = 0, slot_bytes = 0;
+  int nwarp = 0, ring = 0, slot_bytes = 0;
 };
+// Sweep plan of a batch: per member 0 (grid-wide sweep), 1 (one task for the system) or 2 (tasks of
+// preconditioner blocks); the tasks, the chunks of their levels, the chunks' slice descriptors,
+// and the level slice ranges of the cluster sweeps.
 struct SweepPlan {
   std::vector<char> on_task;
   std::vector<TaskDev> tasks;
@@ -193,6 +192,7 @@ struct SweepPlan {
 };
 void plan_sweep_tasks(const std::vector<System *> &sys, bool mixed, bool has_pc, int64_t num_sms, SweepPlan &plan, bool local = true);
 
+// Several systems solved together.
 struct Batch {
   std::vector<System *> sys;
   int nsys = 0;
@@ -220,7 +220,7 @@ struct Batch {
   // streams (trsv_stream.cu) unless vshe_set_task_sweep names a kernel for all
   int nrest = 0;
   struct LocalTables {
-    int tasks = 0, nwarp = 0, ring = 0, slots = 0, slot_bytes = 0;
+    int tasks = 0, nwarp = 0, ring = 0, slot_bytes = 0;
     void *d_tasks = nullptr, *d_runs = nullptr, *d_warps = nullptr, *d_recs = nullptr, *d_buf = nullptr;
     std::vector<int64_t> rec0;
     bool filled = false;  // the records hold the members' present factors

@@ -1263,7 +1263,7 @@ static void add_local_task(const std::vector<System *> &sys, int vb, SweepPlan &
     L.warps.push_back(LocWarp{L.bytes, int32_t(chunks.size()), {bytes(0), bytes(1), bytes(2)}});
     for (size_t h = 0, i = 0; h < chunks.size(); ++h) {
       LocRec R{L.bytes, -1, 0, 0, 0, {}};
-      const LocChunk C{int32_t(chunks[h].first - i), bytes(h + size_t(L.slots) - 1), {0, 0}};
+      const LocChunk C{int32_t(chunks[h].first - i), bytes(h + kLocSlots - 1), {0, 0}};
       static_assert(sizeof(C) == sizeof(R.head), "");
       std::memcpy(&R.head, &C, sizeof(C));
       L.recs.push_back(R);
@@ -1355,8 +1355,7 @@ static void plan_local_tasks(const std::vector<System *> &sys, bool mixed, bool 
   const int64_t left = kLocSmemMax - 8 * int64_t(L.ring) - 128;
   const int64_t want = std::max<int64_t>(1, int64_t(std::ceil(1.5 * slices / std::max(levels, 1.0))));
   L.nwarp = int(std::min<int64_t>(want, kLocWarps));
-  L.slots = kLocSlots;
-  L.slot_bytes = int(std::min<int64_t>(left / (L.slots * L.nwarp), 8192) & ~int64_t(15));
+  L.slot_bytes = int(std::min<int64_t>(left / (kLocSlots * L.nwarp), 8192) & ~int64_t(15));
   // the tasks of a member one after the other, so that its records are one run
   for (size_t k = 0; k < sys.size(); ++k) {
     for (int t = P.nrest; t < P.nrest + P.nlocal; ++t)
@@ -2006,7 +2005,7 @@ int Batch::build_local(Ctx &ctx, const SweepPlan &plan) {
   std::vector<void *> num(sys.size(), nullptr);
   if (plan.nlocal) {
     local.tasks = plan.nlocal;
-    local.nwarp = L.nwarp; local.ring = L.ring; local.slots = L.slots; local.slot_bytes = L.slot_bytes;
+    local.nwarp = L.nwarp; local.ring = L.ring; local.slot_bytes = L.slot_bytes;
     local.rec0 = L.rec0;
     local.d_tasks = table(L.tasks);
     local.d_warps = table(L.warps);
@@ -2224,7 +2223,7 @@ int Batch::launch_tasks(Ctx &ctx, int which) {
   int rc = 0;
   if (nrest) rc = launch_task_kernel(ctx, nrest, which, s);
   if (!rc && local.tasks)
-    rc = vk_trsv_local(mixed ? 1 : 0, local.tasks, local.nwarp, local.ring, local.slots, local.slot_bytes, d_sysdev, d_state, d_active,
+    rc = vk_trsv_local(mixed ? 1 : 0, local.tasks, local.nwarp, local.ring, local.slot_bytes, d_sysdev, d_state, d_active,
                        local.d_tasks, local.d_runs, local.d_warps, local.d_buf, which, d_bar, d_err, s);
   if (!rc && streams.tasks)
     rc = vk_trsv_stream(mixed ? 1 : 0, streams.tasks, streams.nwarp, streams.smem, d_sysdev, d_state, d_active, streams.d_tasks, which, d_bar,
@@ -3124,7 +3123,7 @@ int vshe_layout_local_plan(int64_t n, int64_t nnz, const int64_t *rp, const int3
   plan_sweep_tasks(std::vector<System *>{&S}, S.mixed, S.has_pc, num_sms > 0 ? num_sms : 148, P);
   const LocalPlan &Q = P.local;
   const int64_t c[10] = {int64_t(Q.tasks.size()), int64_t(Q.warps.size()), int64_t(Q.recs.size()), Q.bytes, Q.nwarp, Q.ring,
-                        Q.slots, Q.slot_bytes, P.nrest, int64_t(Q.runs.size())};
+                        kLocSlots, Q.slot_bytes, P.nrest, int64_t(Q.runs.size())};
   std::copy(c, c + 10, counts);
   if (tasks)
     for (size_t t = 0; t < Q.tasks.size(); ++t) {

@@ -63,7 +63,7 @@ VK_DECL_P(double, f64)
 // the apply of block tasks whose solved values fit shared memory (trsv_local.cu), and the fill of one
 // system's records (sysdev: the host's SysDev): all = 1 everything, with the rows' numbers num, 0 the
 // factor's values
-int vk_trsv_local(int mixed, int ntasks, int nwarp, int ring, int slots, int slot_bytes, const void *sys, const void *st, const int32_t *act,
+int vk_trsv_local(int mixed, int ntasks, int nwarp, int ring, int slot_bytes, const void *sys, const void *st, const int32_t *act,
                   const void *tasks, const void *runs, const void *warps, const void *recs, int which, const unsigned *bar, int32_t *err,
                   cudaStream_t s);
 int vk_local_fill(int mixed, const void *sysdev, int nrec, const void *recs, const int32_t *num, int ring, int all, void *buf, cudaStream_t s);

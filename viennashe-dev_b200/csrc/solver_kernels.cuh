@@ -146,15 +146,15 @@ inline constexpr int64_t task_chunk_bytes(int64_t ns, int64_t nslot, int64_t r0,
 // rows are consecutive); entry i of shared memory holds row i's input, then its forward and then its
 // backward result, each in the place of the one before.
 // The slices of a level are dealt to the task's warps by width, and a barrier ends every level.  Every warp
-// has its own sequence of records in chunks, which it copies itself into a ring of `slots`
-// shared-memory slots, slots - 1 chunks ahead.  A chunk is a LocChunk and records one after the other;
+// has its own sequence of records in chunks, which it copies itself into a ring of kLocSlots
+// shared-memory slots, kLocSlots - 1 chunks ahead.  A chunk is a LocChunk and records one after the other;
 // a record is up to kLocCols columns of a slice, four to a group:
 //   LocHead; per group P v[32][4] (factor values), then per group uint16 at[32][4] (numbers of the
 //   values they multiply, `ring` = a zero for padding); the last record of a backward slice also P
 //   dinv[32] (inverse diagonals), uint16 loc[32] (its rows' numbers).
 // k_local_fill writes them from the SELL slices (the values anew after every factorisation).
 struct LocChunk {
-  int32_t nrec, bytes_ahead;  // records; size of the chunk slots - 1 further on (0: none)
+  int32_t nrec, bytes_ahead;  // records; size of the chunk kLocSlots - 1 further on (0: none)
   int32_t pad[2];
 };
 struct LocHead {

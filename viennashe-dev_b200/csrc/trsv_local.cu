@@ -86,7 +86,7 @@ struct Record {
 template <typename P>
 __global__ void __launch_bounds__(32 * kLocWarps, 1)
     k_trsv_local(const SysDev<P> *sys, const BiState *st, const int32_t *active, const LocTask *tasks, const LocRun *runs, const LocWarp *warps,
-                 const unsigned char *recs, int which, int ring, int slots, int slot_bytes, const unsigned *bar, int32_t *err) {
+                 const unsigned char *recs, int which, int ring, int slot_bytes, const unsigned *bar, int32_t *err) {
   __shared__ __align__(8) uint64_t full[kLocWarps * kLocSlots];
   const LocTask T = tasks[blockIdx.x];
   const int s = T.sys;
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(32 * kLocWarps, 1)
   double *val = (double *)l_smem;
   const LocWarp W = warps[T.warp0 + warp];
   uint64_t *mine = full + warp * kLocSlots;
-  unsigned char *slot0 = l_smem + 8 * (size_t)ring + 128 + (size_t)(warp * slots) * slot_bytes;
+  unsigned char *slot0 = l_smem + 8 * (size_t)ring + 128 + (size_t)(warp * kLocSlots) * slot_bytes;
   const unsigned long long limit = spin_limit_of(bar);
   const unsigned char *next = recs + W.off;  // lane 0: the next chunk to copy
   int issued = 0;
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(32 * kLocWarps, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < kLocSlots - 1; ++i)
-      if (i < slots - 1 && i < W.nchunk) issue(i, W.bytes[i]);
+      if (i < W.nchunk) issue(i, W.bytes[i]);
   }
   // the input in the order of the numbers; a lane holds one level's run of rows
   const double *in = which == 0 ? S.p : S.s;
@@ -146,14 +146,14 @@ __global__ void __launch_bounds__(32 * kLocWarps, 1)
   auto give_up = [&]() {
     for (; passed < T.nlev; ++passed) consumers_sync(threads);
     if (lane == 0)
-      for (int q = chunk; q < issued; ++q) mbar_drain(&mine[q % slots], (q / slots) & 1);
+      for (int q = chunk; q < issued; ++q) mbar_drain(&mine[q % kLocSlots], (q / kLocSlots) & 1);
     __syncwarp();
     asm volatile("exit;");
   };
   auto load = [&](Record<P> &R) {
     if (left == 0) {
       if (++chunk == W.nchunk) return false;
-      if (++slot == slots) { slot = 0; phase ^= 1; }
+      if (++slot == kLocSlots) { slot = 0; phase ^= 1; }
       if (!mbar_wait_warp(&mine[slot], phase, limit, err)) give_up();
       rec = slot0 + slot * slot_bytes;
       const LocChunk C = *(const LocChunk *)rec;
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(32 * kLocWarps, 1)
   // the copy that opening a chunk asks for: the slot before it is free, its last record is done
   auto copy_ahead = [&]() {
     if (ahead) {
-      if (lane == 0) issue(slot == 0 ? slots - 1 : slot - 1, ahead);
+      if (lane == 0) issue(slot == 0 ? kLocSlots - 1 : slot - 1, ahead);
       ahead = 0;
     }
   };
@@ -243,15 +243,15 @@ __global__ void k_local_fill(SysDev<P> S, int nrec, const LocRec *recs, const in
 using namespace vshe;
 
 template <typename P>
-static int launch_local(int ntasks, int nwarp, int ring, int slots, int slot_bytes, const void *sys, const void *st, const int32_t *act,
+static int launch_local(int ntasks, int nwarp, int ring, int slot_bytes, const void *sys, const void *st, const int32_t *act,
                         const void *tasks, const void *runs, const void *warps, const void *recs, int which, const unsigned *bar,
                         int32_t *err, cudaStream_t s) {
   cudaError_t e = cudaFuncSetAttribute((const void *)k_trsv_local<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLocSmemMax);
   if (e != cudaSuccess) return (int)e;
   vk_count_launches(1);
-  k_trsv_local<P><<<ntasks, 32 * nwarp, 8 * ring + 128 + nwarp * slots * slot_bytes, s>>>(
+  k_trsv_local<P><<<ntasks, 32 * nwarp, 8 * ring + 128 + nwarp * kLocSlots * slot_bytes, s>>>(
       (const SysDev<P> *)sys, (const BiState *)st, act, (const LocTask *)tasks, (const LocRun *)runs, (const LocWarp *)warps,
-      (const unsigned char *)recs, which, ring, slots, slot_bytes, bar, err);
+      (const unsigned char *)recs, which, ring, slot_bytes, bar, err);
   return (int)cudaGetLastError();
 }
 
@@ -265,11 +265,11 @@ static int launch_local_fill(const void *sysdev, int nrec, const void *recs, con
 
 extern "C" {
 
-int vk_trsv_local(int mixed, int ntasks, int nwarp, int ring, int slots, int slot_bytes, const void *sys, const void *st, const int32_t *act,
+int vk_trsv_local(int mixed, int ntasks, int nwarp, int ring, int slot_bytes, const void *sys, const void *st, const int32_t *act,
                   const void *tasks, const void *runs, const void *warps, const void *recs, int which, const unsigned *bar, int32_t *err,
                   cudaStream_t s) {
-  return mixed ? launch_local<float>(ntasks, nwarp, ring, slots, slot_bytes, sys, st, act, tasks, runs, warps, recs, which, bar, err, s)
-               : launch_local<double>(ntasks, nwarp, ring, slots, slot_bytes, sys, st, act, tasks, runs, warps, recs, which, bar, err, s);
+  return mixed ? launch_local<float>(ntasks, nwarp, ring, slot_bytes, sys, st, act, tasks, runs, warps, recs, which, bar, err, s)
+               : launch_local<double>(ntasks, nwarp, ring, slot_bytes, sys, st, act, tasks, runs, warps, recs, which, bar, err, s);
 }
 
 int vk_local_fill(int mixed, const void *sysdev, int nrec, const void *recs, const int32_t *num, int ring, int all, void *buf, cudaStream_t s) {
