@@ -129,7 +129,8 @@ void vshe_default_opts(vshe_solve_opts *opts);
 /* ---- context ---- */
 typedef struct vshe_ctx vshe_ctx;
 
-/* Creates a context on CUDA device `device`; hbm_budget_bytes = 0 means 150 GB. */
+/* Creates a context on CUDA device `device`; hbm_budget_bytes = 0 means 150 GB.  Copies of the factors that
+ * make sweeps sooner are kept within what the systems leave of it, and give way to later systems. */
 int vshe_create(vshe_ctx **ctx, int device, size_t hbm_budget_bytes);
 int vshe_destroy(vshe_ctx *ctx);
 const char *vshe_errstr(int code);
@@ -153,9 +154,9 @@ int vshe_set_spin_limit(vshe_ctx *ctx, uint64_t polls);
 int vshe_set_host_threads(int32_t threads);
 /* Sweep kernel of the members swept one task per CTA or cluster (VSHE_TRSV_PER_BLOCK,
  * VSHE_TRSV_PER_SYSTEM and their AUTO cases): -1 (default) takes the kernels that keep the solved
- * values in shared memory for whole systems and for block tasks whose rows fit it, and for the other
- * tasks times the candidates on each batch's own factors before its first iteration and keeps the
- * fastest; 0 one CTA per task with the factor slices staged through shared memory by bulk copies; 2, 4
+ * values in shared memory for whole systems and block tasks that fit it where these are the sooner, and
+ * for the other tasks times the candidates on each batch's own factors before its first iteration and
+ * keeps the fastest; 0 one CTA per task with the factor slices staged through shared memory by bulk copies; 2, 4
  * or 8 one thread-block cluster of that many CTAs per task with a cluster barrier per level.  Every
  * choice gives bitwise the same results.  No reference counterpart: scheduling control of the
  * triangular sweeps. */

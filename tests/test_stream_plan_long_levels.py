@@ -41,3 +41,13 @@ def test_level_of_several_chunks(long, width, precision):
         plans.test_stream_runs_like_the_level_sweep("long level")
     finally:
         del plans.STREAMS["long level"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("long", [4000, 7000, 8000, 8193])
+def test_same_x_as_task(long, precision):
+    import test_gpu_local_sweeps as sweeps
+    rp, ci, v, _ = _levels([600] * 16 + [long] + [600] * 16, 3)
+    b = np.random.default_rng(1).uniform(-1.0, 1.0, len(rp) - 1)
+    assert sweeps._both((rp, ci, v, b), precision, **dict(plans.NAT, trsv="per_system")) == 3

@@ -84,9 +84,11 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_al
 // entries is summed by its warp instead, lanes striding it, so that it does not wait on one thread,
 // whatever the rows around it.  Before, a warp walked a row at a time and 256 rows in series
 // (10 of its 32 lanes busy, three dependent loads a row).  Rows of 9 entries, before and now:
-// 1000 rows 94 and 6.3 us, 100 003 rows 199 and 10.3 us, 1 000 003 rows 310 and 42.6 us
-// (3.5 TB/s), 8 M rows 1271 and 290 us (4.1 TB/s).  Tiles of 256 rows, three blocks an SM: 49 and
-// 329 us on the last two; one buffer instead of two: 48 and 329 us.
+// 1000 rows 94 and 6.5 us, 100 003 rows 199 and 10.4 us, 1 000 003 rows 301 and 41.2 us
+// (3.4 TB/s), 8 M rows 1271 and 277 us (4.0 TB/s).  With one running sum a row, and 42.7 and 293 us on the
+// last two: tiles of 256 rows, three blocks an SM 49 and 329 us; one buffer instead of two 48 and 329 us.
+// L2 flushed, rows of 8 with one of 3000 in 128 937 and 59 us (200 000 rows), rows of 33 to 47 370 and
+// 121 us (500 000 rows).
 // The last block to finish adds the block partials in block order; the order of every sum is fixed
 // by the matrix and the SM count.
 // Four partial sums are no less accurate than a warp that strides the row and adds its lanes up in a tree
