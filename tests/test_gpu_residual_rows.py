@@ -54,62 +54,6 @@ def test_edges(gpu_ctx, n, kind):
     assert np.all(np.abs(n2 - want) <= 1e-12 * want)
 
 
-"""vshe_csr_residual_noalloc by row length: tiles and chunks at their edges (128 rows, 1536 entries, one
-tile for every resident block and one more), and the rounding of a row's sum.  The sums may be no less
-accurate than one warp striding the row and adding its lanes up in a tree, the plainest order for a
-CSR row: root mean square error against extended precision at most 3 % above that order's in numpy (the
-means of 20000 rows scatter by 0.5 % each).  Reference of the edges: numpy in extended precision, each row
-within its rounding bound, (entries + 2) eps (|b| + sum |a||x|)."""
-import ctypes as C
-
-import numpy as np
-import pytest
-
-from vshe import gpu
-
-pytestmark = pytest.mark.gpu
-LD = np.longdouble
-
-
-def _residual(rp, ci, v, x, b):
-    import torch
-    dev = [torch.from_numpy(a).to("cuda") for a in (rp, ci, v, x, b)]
-    r, n2 = torch.full_like(dev[4], float("nan")), torch.full((2,), float("nan"), dtype=torch.float64, device="cuda")
-    torch.cuda.synchronize()
-    L = gpu.lib()
-    L.vshe_csr_residual_noalloc.argtypes = [C.c_int64, C.c_int64] + [C.c_void_p] * 8
-    assert L.vshe_csr_residual_noalloc(len(b), len(ci), *[a.data_ptr() for a in dev], r.data_ptr(), n2.data_ptr(), None) == 0
-    torch.cuda.synchronize()
-    return r.cpu().numpy(), n2.cpu().numpy()
-
-
-def _system(lengths, seed=5):
-    rng = np.random.default_rng(seed)
-    n = len(lengths)
-    rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int64)
-    return rp, rng.integers(0, n, rp[-1]).astype(np.int32), rng.standard_normal(rp[-1]), rng.standard_normal(n), rng.standard_normal(n)
-
-
-@pytest.mark.parametrize("n", [127, 128, 129, 94720, 94721, 2 * 94720 + 1])
-@pytest.mark.parametrize("kind", ["short", "edge", "dense in short", "dense in wide"])
-def test_edges(gpu_ctx, n, kind):
-    rng = np.random.default_rng(n)
-    k = rng.integers(0, 13, n) if kind != "dense in wide" else rng.integers(33, 70, n)
-    if kind == "edge":  # around the longest row of one thread, in a tile of more than a chunk
-        k[:128] = 12
-        k[[5, 40, 41, 90]] = [47, 48, 49, 50]
-    elif kind != "short":
-        k[n // 3], k[n - 1], k[1] = 3000, 1537, 1536
-    rp, ci, v, x, b = _system(k)
-    r, n2 = _residual(rp, ci, v, x, b)
-    prod = v.astype(LD) * x[ci]
-    cs, mag = np.concatenate([[0], np.cumsum(prod)]), np.concatenate([[0], np.cumsum(np.abs(prod))])
-    bound = (k + 2) * np.finfo(float).eps * (np.abs(b) + (mag[rp[1:]] - mag[rp[:-1]])) + 1e-17 * mag[-1]
-    assert np.all(np.abs(r - (b - (cs[rp[1:]] - cs[rp[:-1]]))) <= bound)
-    want = np.array([np.sum(r.astype(LD) ** 2), np.sum(b.astype(LD) ** 2)], np.float64)
-    assert np.all(np.abs(n2 - want) <= 1e-12 * want)
-
-
 def _warp_sums(v, x):
     acc = np.zeros((len(v), 32))
     for k in range(v.shape[1]):
